@@ -11,6 +11,7 @@
 #include <cstring>
 #include <mutex>
 #include <new>
+#include <type_traits>
 #include <unordered_map>
 #include <vector>
 
@@ -19,6 +20,7 @@
 #include "decode.cuh"
 #include "diag.hpp"
 #include "gemm.cuh"
+#include "gemm_rows.cuh"
 #include "rms_norm.cuh"
 
 using x17::make_diag;
@@ -28,7 +30,7 @@ namespace {
 
 std::atomic<uint64_t> g_launches{0};
 std::atomic<int> g_attn_schedule{X17AI_B200_ATTN_PER_TILE};
-std::atomic<int> g_gemm_tiling{X17AI_B200_GEMM_CTA_PAIR};
+std::atomic<int> g_gemm_tiling{X17AI_B200_GEMM_AUTO};
 std::atomic<unsigned> g_attn_item_tiles{0};   // 0 = chosen per launch
 std::mutex g_capture_mutex;
 std::unordered_map<void *, CUcontext> g_capture_ctx;   // streams between graph_begin and graph_end
@@ -438,8 +440,6 @@ void fill_gemm_params(x17ai_GemmConfig const *cfg, GemmPlan const &plan, size_t 
 	}
 }
 
-// The CTA-pair form (gemm.cuh): clusters of two CTAs, one 256 x 256 tile per cluster. `tb_half` is B's map with a box
-// of half a tile's rows. Used for more than one row tile when the tiling is X17AI_B200_GEMM_CTA_PAIR.
 // How many clusters of the pair kernel the device runs at once. The kernel is persistent, so the grid must not be
 // larger: a cluster needs two free SMs of one GPC, and a GPU whose GPCs have an odd number of usable SMs holds fewer
 // pairs than sm_count / 2; a cluster left over would run alone after all the others. Asked once per kernel and
@@ -474,7 +474,7 @@ uint32_t max_pair_clusters(Kernel kernel, uint32_t smem, int sm_count) {
 }
 
 // The CTA-pair form (gemm.cuh): clusters of two CTAs, one 256 x 256 tile per cluster. `tb_half` is B's map with a box
-// of half a tile's rows. Used for more than one row tile when the tiling is X17AI_B200_GEMM_CTA_PAIR.
+// of half a tile's rows. Used for more than one row tile unless the tiling is X17AI_B200_GEMM_ONE_CTA.
 template <int EPI, bool F8>
 cudaError_t gemm_go_pair_kind(int sm_count, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tb_half,
 							  x17::GemmParams const &p) {
@@ -493,6 +493,150 @@ cudaError_t gemm_go_pair(bool f8, int sm_count, cudaStream_t stream, CUtensorMap
 						 x17::GemmParams const &p) {
 	return f8 ? gemm_go_pair_kind<EPI, true>(sm_count, stream, ta, tb_half, p)
 			  : gemm_go_pair_kind<EPI, false>(sm_count, stream, ta, tb_half, p);
+}
+
+// The form for few rows (gemm.cuh): a cluster of up to four CTAs shares one 128 x 256 tile, K split over it.
+// Taken (default tiling only) for up to 128 rows, where a persistent form has one CTA per column tile at most, and
+// for more rows while the CTA-pair form's tiles would keep no more than half of the SMs busy and K is long enough
+// (4096) to pay for the exchange of the parts.
+struct SplitPlan {
+	x17::SplitParams sp{};
+	uint32_t grid = 0, smem = 0;
+	explicit operator bool() const { return grid != 0; }
+};
+// Deals the chunks of a plain tile and of a tile of heads out to the CTAs; returns the most that one CTA gets.
+uint32_t deal_chunks(x17::SplitParams &sp, uint32_t head_dim) {
+	using namespace x17::gemm_cfg;
+	uint32_t most = 0;
+	for (int heads_tile = 0; heads_tile < (head_dim != 0 ? 2 : 1); ++heads_tile) {
+		uint32_t count[SPLIT_MAX] = {};
+		sp.owner[heads_tile] = sp.before[heads_tile] = 0;
+		uint32_t const half = head_dim / 32, heads = heads_tile ? SPLIT_CHUNKS / (2 * half) : 0;
+		for (uint32_t c = 0; c < SPLIT_CHUNKS; ++c) {
+			uint32_t o = c % sp.split;
+			if (heads_tile) {
+				uint32_t const head = c / (2 * half), i = c % (2 * half), v = head * half + i - half;
+				o = i < half ? head % sp.split : heads < sp.split ? heads + v % (sp.split - heads) : (heads + v) % sp.split;
+			}
+			sp.owner[heads_tile] |= o << (4 * c);
+			sp.before[heads_tile] |= count[o] << (4 * c);
+			most = ++count[o] > most ? count[o] : most;
+		}
+	}
+	return most;
+}
+SplitPlan plan_split(size_t rows, size_t n_raw, size_t k, uint32_t head_dim, int sm_count) {
+	using namespace x17::gemm_cfg;
+	SplitPlan plan;
+	if (g_gemm_tiling.load(std::memory_order_relaxed) != X17AI_B200_GEMM_AUTO) return plan;
+	size_t const tiles_n = (n_raw + BN - 1) / BN, pair_tiles = ((rows + 2 * BM - 1) / (2 * BM)) * tiles_n;
+	size_t const tiles_m = (rows + BM - 1) / BM, tiles = tiles_m * tiles_n, k_blocks = k / BK;
+	if (rows > BM && (4 * pair_tiles > size_t(sm_count) || k_blocks < 32)) return plan;
+	if (tiles > (size_t(1) << 27)) return plan;
+	x17::SplitParams &sp = plan.sp;
+	sp.tiles_m = uint32_t(tiles_m);
+	sp.a_rows = rows >= BM ? BM : uint32_t((rows + 7) / 8 * 8);
+	// three stages of up to 36 KB leave room for two CTAs per SM
+	sp.stages = sp.a_rows <= 32 ? 3 : SPLIT_MAX_STAGES;
+	// as many CTAs per tile as the SMs hold (clusters of three, or of eight, leave SMs of a GPC unused: a second wave),
+	// each with two K blocks or more (eight where whole heads are finished by one CTA)
+	size_t const least = head_dim != 0 ? 8 : 2;
+	size_t split = SPLIT_MAX;
+	while (split > 1 && (tiles * split > size_t(sm_count) || k_blocks / split < least)) split /= 2;
+	// the parts of the other CTAs land in the ring
+	for (;; split /= 2) {
+		sp.split = uint32_t(split);
+		sp.slots = deal_chunks(sp, head_dim);
+		if (split == 1 || (split - 1) * sp.slots * sp.a_rows * 128 <= size_t(sp.stages) * (sp.a_rows * BK + B_BYTES)) break;
+	}
+	plan.grid = uint32_t(tiles * split);
+	plan.smem = split_smem_bytes(sp.a_rows, sp.stages);
+	return plan;
+}
+
+template <int EPI, bool F8>
+cudaError_t gemm_go_split_kind(SplitPlan const &plan, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tb,
+							   x17::GemmParams const &p) {
+	auto const kernel = x17::gemm_split_kernel<EPI, F8>;
+	using namespace x17::gemm_cfg;
+	cudaError_t const ce = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+												int(split_smem_bytes(BM, SPLIT_MAX_STAGES)));
+	if (ce != cudaSuccess) return ce;
+	cudaLaunchAttribute attr{};
+	attr.id = cudaLaunchAttributeClusterDimension;
+	attr.val.clusterDim.x = plan.sp.split;
+	attr.val.clusterDim.y = 1;
+	attr.val.clusterDim.z = 1;
+	cudaLaunchConfig_t cfg{};
+	cfg.gridDim = dim3(plan.grid);
+	cfg.blockDim = dim3(THREADS);
+	cfg.dynamicSmemBytes = plan.smem;
+	cfg.stream = stream;
+	cfg.attrs = &attr;
+	cfg.numAttrs = 1;
+	return cudaLaunchKernelEx(&cfg, kernel, ta, tb, p, plan.sp);
+}
+template <int EPI>
+cudaError_t gemm_go_split(bool f8, SplitPlan const &plan, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tb,
+						  x17::GemmParams const &p) {
+	return f8 ? gemm_go_split_kind<EPI, true>(plan, stream, ta, tb, p) : gemm_go_split_kind<EPI, false>(plan, stream, ta, tb, p);
+}
+
+// The form for up to 48 rows (gemm_rows.cuh; above that its L2 -> SM traffic, the tokens' bytes once per 128 columns,
+// costs more than the 256-column tiles of the split form save: at 64 rows the e4m3 x int8 projection of
+// [8192, 2 x 14336] takes 54 us against 45). K is split over a cluster of up to four CTAs as long as all CTAs run at
+// once, two to an SM, and each has four K blocks or more.
+struct RowsPlan {
+	x17::RowsParams rp{};
+	uint32_t grid = 0, smem = 0;
+	explicit operator bool() const { return grid != 0; }
+};
+RowsPlan plan_rows(size_t rows, size_t n_raw, size_t k, bool heads, int sm_count) {
+	using namespace x17::rows_cfg;
+	RowsPlan plan;
+	if (g_gemm_tiling.load(std::memory_order_relaxed) != X17AI_B200_GEMM_AUTO || rows > MAX_TOK) return plan;
+	size_t const tiles = n_raw / WM, k_blocks = k / BK;
+	if (tiles > (size_t(1) << 27)) return plan;
+	x17::RowsParams &rp = plan.rp;
+	rp.a_box = uint32_t((rows + 7) / 8 * 8);
+	rp.n_tok = uint32_t((rows + 15) / 16 * 16);
+	constexpr uint32_t BUDGET = 110 * 1024;   // two CTAs per SM
+	rp.stages = BUDGET / stage_bytes(rp.a_box);
+	if (rp.stages > MAX_STAGES) rp.stages = MAX_STAGES;
+	rp.split = 4;
+	while (rp.split > 1 && (tiles * rp.split > 2 * size_t(sm_count) || k_blocks / rp.split < 4
+							|| tail_bytes(rp.split, rp.n_tok, heads) > rp.stages * stage_bytes(rp.a_box))) {
+		rp.split /= 2;
+	}
+	plan.grid = uint32_t(tiles) * rp.split;
+	plan.smem = smem_bytes(rp.a_box, rp.stages);
+	return plan;
+}
+
+template <int EPI, bool F8>
+cudaError_t gemm_go_rows_kind(RowsPlan const &plan, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tw,
+							  x17::GemmParams const &p) {
+	auto const kernel = x17::gemm_rows_kernel<EPI, F8>;
+	cudaError_t const ce = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
+	if (ce != cudaSuccess) return ce;
+	cudaLaunchAttribute attr{};
+	attr.id = cudaLaunchAttributeClusterDimension;
+	attr.val.clusterDim.x = plan.rp.split;
+	attr.val.clusterDim.y = 1;
+	attr.val.clusterDim.z = 1;
+	cudaLaunchConfig_t cfg{};
+	cfg.gridDim = dim3(plan.grid);
+	cfg.blockDim = dim3(x17::rows_cfg::THREADS);
+	cfg.dynamicSmemBytes = plan.smem;
+	cfg.stream = stream;
+	cfg.attrs = &attr;
+	cfg.numAttrs = 1;
+	return cudaLaunchKernelEx(&cfg, kernel, ta, tw, p, plan.rp);
+}
+template <int EPI>
+cudaError_t gemm_go_rows(bool f8, RowsPlan const &plan, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tw,
+						 x17::GemmParams const &p) {
+	return f8 ? gemm_go_rows_kind<EPI, true>(plan, stream, ta, tw, p) : gemm_go_rows_kind<EPI, false>(plan, stream, ta, tw, p);
 }
 
 template <int EPI>
@@ -823,7 +967,7 @@ int x17ai_b200_set_attn_schedule(int schedule, unsigned tiles_per_item) {
 }
 
 int x17ai_b200_set_gemm_tiling(int tiling) {
-	if (tiling != X17AI_B200_GEMM_ONE_CTA && tiling != X17AI_B200_GEMM_CTA_PAIR) return -1;
+	if (tiling < X17AI_B200_GEMM_ONE_CTA || tiling > X17AI_B200_GEMM_AUTO) return -1;
 	g_gemm_tiling.store(tiling, std::memory_order_relaxed);
 	return 0;
 }
@@ -1141,10 +1285,13 @@ x17ai_DiagnosticBuffer *x17ai_b200_gemm_fwd(
 	size_t const k_a = cfg->a_cols;
 	size_t const k_total = plan.split ? 2 * k_a : k_a;
 	CUtensorMap ta, tb;
-	bool const pair = g_gemm_tiling.load(std::memory_order_relaxed) == X17AI_B200_GEMM_CTA_PAIR && a_rows > BM
+	RowsPlan const few = plan_rows(a_rows, cfg->b_rows, k_total, plan.epi == x17::EPI_L2NORM_KV, scope.state().sm_count);
+	SplitPlan const split = plan_split(a_rows, cfg->b_rows, k_total, plan.epi == x17::EPI_L2NORM_KV ? uint32_t(cfg->head_dim) : 0u,
+									   scope.state().sm_count);
+	bool const pair = !split && g_gemm_tiling.load(std::memory_order_relaxed) != X17AI_B200_GEMM_ONE_CTA && a_rows > BM
 					  && cfg->b_rows % BN == 0 && scope.state().sm_count >= 2;
-	CUresult e = make_map_2d(&ta, a, k_a, a_rows, k_a, BK, BM);
-	if (e == CUDA_SUCCESS) e = make_map_2d(&tb, b, k_total, cfg->b_rows, k_total, BK, pair ? BN / 2 : BN);
+	CUresult e = make_map_2d(&ta, a, k_a, a_rows, k_a, BK, few ? few.rp.a_box : split ? split.sp.a_rows : BM);
+	if (e == CUDA_SUCCESS) e = make_map_2d(&tb, b, k_total, cfg->b_rows, k_total, BK, few || pair ? BN / 2 : BN);
 	if (e != CUDA_SUCCESS) {
 		return make_diag("x17ai_b200: cuTensorMapEncodeTiled failed", who,
 						 ": cuTensorMapEncodeTiled failed: ", x17::cu_error_text(e));
@@ -1160,24 +1307,20 @@ x17ai_DiagnosticBuffer *x17ai_b200_gemm_fwd(
 	dim3 grid(ctas);
 	cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
 	cudaError_t ce;
-	if (pair) {
-		int const sms = scope.state().sm_count;
-		switch (plan.epi) {
-		case x17::EPI_SCALE_I8: ce = gemm_go_pair<x17::EPI_SCALE_I8>(plan.f8, sms, s, ta, tb, p); break;
-		case x17::EPI_RAW_I32: ce = gemm_go_pair<x17::EPI_RAW_I32>(plan.f8, sms, s, ta, tb, p); break;
-		case x17::EPI_L2NORM_KV: ce = gemm_go_pair<x17::EPI_L2NORM_KV>(plan.f8, sms, s, ta, tb, p); break;
-		case x17::EPI_GEGLU_E4M3: ce = gemm_go_pair<x17::EPI_GEGLU_E4M3>(plan.f8, sms, s, ta, tb, p); break;
-		case x17::EPI_RESID_E4M3: ce = gemm_go_pair<x17::EPI_RESID_E4M3>(plan.f8, sms, s, ta, tb, p); break;
-		default: ce = gemm_go_pair<x17::EPI_RESID_I8>(plan.f8, sms, s, ta, tb, p); break;
-		}
-	} else
+	auto go = [&](auto epi) {
+		constexpr int EPI = decltype(epi)::value;
+		if (few) return gemm_go_rows<EPI>(plan.f8, few, s, ta, tb, p);
+		if (split) return gemm_go_split<EPI>(plan.f8, split, s, ta, tb, p);
+		if (pair) return gemm_go_pair<EPI>(plan.f8, scope.state().sm_count, s, ta, tb, p);
+		return gemm_go<EPI>(plan.f8, grid, s, ta, tb, p);
+	};
 	switch (plan.epi) {
-	case x17::EPI_SCALE_I8: ce = gemm_go<x17::EPI_SCALE_I8>(plan.f8, grid, s, ta, tb, p); break;
-	case x17::EPI_RAW_I32: ce = gemm_go<x17::EPI_RAW_I32>(plan.f8, grid, s, ta, tb, p); break;
-	case x17::EPI_L2NORM_KV: ce = gemm_go<x17::EPI_L2NORM_KV>(plan.f8, grid, s, ta, tb, p); break;
-	case x17::EPI_GEGLU_E4M3: ce = gemm_go<x17::EPI_GEGLU_E4M3>(plan.f8, grid, s, ta, tb, p); break;
-	case x17::EPI_RESID_E4M3: ce = gemm_go<x17::EPI_RESID_E4M3>(plan.f8, grid, s, ta, tb, p); break;
-	default: ce = gemm_go<x17::EPI_RESID_I8>(plan.f8, grid, s, ta, tb, p); break;
+	case x17::EPI_SCALE_I8: ce = go(std::integral_constant<int, x17::EPI_SCALE_I8>{}); break;
+	case x17::EPI_RAW_I32: ce = go(std::integral_constant<int, x17::EPI_RAW_I32>{}); break;
+	case x17::EPI_L2NORM_KV: ce = go(std::integral_constant<int, x17::EPI_L2NORM_KV>{}); break;
+	case x17::EPI_GEGLU_E4M3: ce = go(std::integral_constant<int, x17::EPI_GEGLU_E4M3>{}); break;
+	case x17::EPI_RESID_E4M3: ce = go(std::integral_constant<int, x17::EPI_RESID_E4M3>{}); break;
+	default: ce = go(std::integral_constant<int, x17::EPI_RESID_I8>{}); break;
 	}
 	if (ce != cudaSuccess) {
 		return make_diag("x17ai_b200: cudaFuncSetAttribute failed", who, ": cudaFuncSetAttribute failed: ",
@@ -1217,10 +1360,12 @@ x17ai_DiagnosticBuffer *x17ai_b200_qkvg_fwd_i8(
 	using namespace x17::gemm_cfg;
 	size_t const n_raw = n_q + n_kv + n_g;
 	CUtensorMap ta, tb;
-	bool const pair = g_gemm_tiling.load(std::memory_order_relaxed) == X17AI_B200_GEMM_CTA_PAIR && rows > BM
+	RowsPlan const few = plan_rows(rows, n_raw, cfg->model_dim, true, scope.state().sm_count);
+	SplitPlan const split = plan_split(rows, n_raw, cfg->model_dim, uint32_t(cfg->head_dim), scope.state().sm_count);
+	bool const pair = !split && g_gemm_tiling.load(std::memory_order_relaxed) != X17AI_B200_GEMM_ONE_CTA && rows > BM
 					  && n_raw % BN == 0 && scope.state().sm_count >= 2;
-	CUresult e = make_map_2d(&ta, x, cfg->model_dim, rows, cfg->model_dim, BK, BM);
-	if (e == CUDA_SUCCESS) e = make_map_2d(&tb, w_qkvg, cfg->model_dim, n_raw, cfg->model_dim, BK, pair ? BN / 2 : BN);
+	CUresult e = make_map_2d(&ta, x, cfg->model_dim, rows, cfg->model_dim, BK, few ? few.rp.a_box : split ? split.sp.a_rows : BM);
+	if (e == CUDA_SUCCESS) e = make_map_2d(&tb, w_qkvg, cfg->model_dim, n_raw, cfg->model_dim, BK, few || pair ? BN / 2 : BN);
 	if (e != CUDA_SUCCESS) {
 		return make_diag("x17ai_b200: cuTensorMapEncodeTiled failed", who,
 						 ": cuTensorMapEncodeTiled failed: ", x17::cu_error_text(e));
@@ -1251,7 +1396,9 @@ x17ai_DiagnosticBuffer *x17ai_b200_qkvg_fwd_i8(
 	uint32_t const n_tiles = p.tiles_m * p.tiles_n;
 	uint32_t const ctas = n_tiles < uint32_t(scope.state().sm_count) ? n_tiles : uint32_t(scope.state().sm_count);
 	cudaError_t const ce =
-		pair ? gemm_go_pair<x17::EPI_QKVG>(false, scope.state().sm_count, reinterpret_cast<cudaStream_t>(stream), ta, tb, p)
+		few ? gemm_go_rows<x17::EPI_QKVG>(false, few, reinterpret_cast<cudaStream_t>(stream), ta, tb, p)
+		: split ? gemm_go_split<x17::EPI_QKVG>(false, split, reinterpret_cast<cudaStream_t>(stream), ta, tb, p)
+		: pair ? gemm_go_pair<x17::EPI_QKVG>(false, scope.state().sm_count, reinterpret_cast<cudaStream_t>(stream), ta, tb, p)
 			 : gemm_go<x17::EPI_QKVG>(false, dim3(ctas), reinterpret_cast<cudaStream_t>(stream), ta, tb, p);
 	if (ce != cudaSuccess) {
 		return make_diag("x17ai_b200: cudaFuncSetAttribute failed", who, ": cudaFuncSetAttribute failed: ",

@@ -80,16 +80,6 @@ constexpr f32 MAGIC = 12582912.0f;  // 1.5 * 2^23
 constexpr u32 MAGIC_BITS = 0x4B400000u;
 }  // namespace attn_cfg
 
-X17_DEV uint4 ld_shared_v4(u32 addr) {
-	uint4 v;
-	asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-	return v;
-}
-X17_DEV void st_shared_v4(u32 addr, u32 a, u32 b, u32 c, u32 d) {
-	asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d)
-				 : "memory");
-}
-
 // N score columns of one row -> probabilities: accumulates the un-rounded exp2 into sum[4] and
 // returns rint(255 * p) packed four to a word. EDGE: only columns lo <= col < lo + span are visible.
 // The four f32 operations per element are issued as packed f32x2 instructions (two elements per

@@ -110,6 +110,87 @@ X17_DEV f32 acc_to_f32(u32 bits) {
 	}
 }
 
+// 32 accumulator columns of one row -> output bytes. `scale32`: FixedI8 codes; `pairs32`: one byte per (even, odd)
+// pair of columns, GeGLU or gated residual (`rw`: the row's 16 residual codes).
+template <bool F8>
+X17_DEV void scale32(u32 const (&r)[32], f32 sc, u32 (&w)[8]) {
+#pragma unroll
+	for (u32 i = 0; i < 8; ++i) {
+		w[i] = pack4(u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 0]), sc))),
+					 u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 1]), sc))),
+					 u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 2]), sc))),
+					 u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 3]), sc))));
+	}
+}
+template <int EPI, bool F8>
+X17_DEV void pairs32(u32 const (&r)[32], u32 const (&rw)[4], GemmParams const &p, u32 (&w)[4]) {
+#pragma unroll
+	for (u32 i = 0; i < 4; ++i) {
+		u32 b[4];
+#pragma unroll
+		for (u32 j = 0; j < 4; ++j) {
+			f32 const gate = acc_to_f32<F8>(r[8 * i + 2 * j]);
+			f32 const val = acc_to_f32<F8>(r[8 * i + 2 * j + 1]);
+			if constexpr (EPI == EPI_GEGLU_E4M3) {
+				b[j] = f32_to_e4m3(geglu_val(gate, val, p));
+			} else {
+				f32 const v = resid_val(gate, val, f32(i32(static_cast<i8>((rw[i] >> (8 * j)) & 0xFFu))), p);
+				b[j] = EPI == EPI_RESID_E4M3 ? f32_to_e4m3(v) : u32(f32_to_fixedi8(v));
+			}
+		}
+		w[i] = pack4(b[0], b[1], b[2], b[3]);
+	}
+}
+X17_DEV void store32(void *dst, u32 const (&w)[8]) {
+	static_cast<uint4 *>(dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+	static_cast<uint4 *>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+}
+// The same for the epilogues that work column by column (everything but the per-head L2 norm): columns
+// [col, col + 32) of `row`.
+template <int EPI, bool F8>
+X17_DEV void store_cols32(u32 const (&r)[32], GemmParams const &p, u32 row, u32 col) {
+	if constexpr (EPI == EPI_SCALE_I8) {   // k0 = f32(inp_scale * out_scale)
+		u32 w[8];
+		scale32<F8>(r, p.k0, w);
+		store32(static_cast<i8 *>(p.c) + u64(row) * p.c_stride + col, w);
+	} else if constexpr (EPI == EPI_RAW_I32) {
+		uint4 *dst = reinterpret_cast<uint4 *>(static_cast<u32 *>(p.c) + u64(row) * p.c_stride + col);
+#pragma unroll
+		for (u32 i = 0; i < 8; ++i) dst[i] = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+	} else {
+		u32 rw[4] = {0, 0, 0, 0};
+		if constexpr (EPI != EPI_GEGLU_E4M3) {
+			uint4 const res = *reinterpret_cast<uint4 const *>(p.residual + u64(row) * p.resid_stride + col / 2);
+			rw[0] = res.x; rw[1] = res.y; rw[2] = res.z; rw[3] = res.w;
+		}
+		u32 w[4];
+		pairs32<EPI, F8>(r, rw, p, w);
+		*reinterpret_cast<uint4 *>(static_cast<u8 *>(p.c) + u64(row) * p.c_stride + col / 2) = make_uint4(w[0], w[1], w[2], w[3]);
+	}
+}
+// Where a tile's columns go in the epilogues with per-head L2 norm: the key/value segment of the fused projection or
+// the whole output, or one of the plain segments (q, g) of the fused projection.
+struct SegOut {
+	i8 *base;
+	u64 stride;
+	u32 col0;    // of the tile inside the segment
+	u32 width;   // columns of the segment
+	f32 scale;   // plain segments, and V
+	bool heads;  // per head [K(D) | V(D)]: K l2-normalised, V scaled
+};
+template <int EPI>
+X17_DEV SegOut segment_of(GemmParams const &p, u32 n0) {
+	if constexpr (EPI == EPI_QKVG) {
+		if (n0 < p.n_q) return {static_cast<i8 *>(p.c), p.c_stride, n0, p.n_q, p.k3, false};
+		if (n0 >= p.n_q + p.n_kv) {
+			return {static_cast<i8 *>(p.c3), p.c3_stride, n0 - p.n_q - p.n_kv, p.n_raw - p.n_q - p.n_kv, p.k4, false};
+		}
+		return {static_cast<i8 *>(p.c2), p.c2_stride, n0 - p.n_q, p.n_kv, p.k2, true};
+	} else {
+		return {static_cast<i8 *>(p.c), p.c_stride, n0, p.n_raw, p.k2, true};
+	}
+}
+
 // ---- kernel ----------------------------------------------------------------------------------
 
 // Tile order of the persistent loop: groups of GROUP_M row tiles; inside a group the row tiles run
@@ -301,113 +382,33 @@ X17_DEV void gemm_body(CUtensorMap const *tm_a_ptr, CUtensorMap const *tm_b_ptr,
 			bool const row_ok = row < p.m;
 			u32 const t_base = tmem_base + buf * ACC_COLS + ((quarter * 32u) << 16);
 
-			if constexpr (EPI == EPI_QKVG) {
-				if (n0 < p.n_q || n0 >= p.n_q + p.n_kv) {
-					// q or g segment: plain scale -> FixedI8 (ScaledMatrixWriter, gemm_b8.cuh:291-339)
-					bool const is_q = n0 < p.n_q;
-					i8 *const base = static_cast<i8 *>(is_q ? p.c : p.c3);
-					u64 const stride = is_q ? p.c_stride : p.c3_stride;
-					u32 const col0 = is_q ? n0 : n0 - p.n_q - p.n_kv;
-					u32 const width = is_q ? p.n_q : p.n_raw - p.n_q - p.n_kv;
-					f32 const sc = is_q ? p.k3 : p.k4;
-					for (u32 c = 0; c < BN && col0 + c < width; c += 32) {
-						u32 r[32];
-						tmem_ld_32x32b_x32(t_base + c, r);
-						tmem_wait_ld();
-						u32 w[8];
-#pragma unroll
-						for (u32 i = 0; i < 8; ++i) {
-							w[i] = pack4(u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 0]), sc))),
-										 u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 1]), sc))),
-										 u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 2]), sc))),
-										 u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 3]), sc))));
-						}
-						if (row_ok) {
-							uint4 *dst = reinterpret_cast<uint4 *>(base + u64(row) * stride + col0 + c);
-							dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-							dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
-						}
-					}
-				} else {
-					// kv segment: per head [K(D) | V(D)] (L2NormMatrixWriter, gemm_b8.cuh:861-949)
-					u32 const d = p.head_dim;
-					u32 const col0 = n0 - p.n_q;
-					for (u32 h0 = 0; h0 < BN && col0 + h0 < p.n_kv; h0 += 2 * d) {
+			if constexpr (EPI == EPI_QKVG || EPI == EPI_L2NORM_KV) {
+				// k0 = eps, k1 = HEAD_SCALE (= out_scale * sqrt(D)), k2 = SEP_SCALE (= inp * out)
+				SegOut const seg = segment_of<EPI>(p, n0);
+				u32 const d2 = seg.heads ? 2 * p.head_dim : 32u;   // columns that are written under one scale pair
+				for (u32 h0 = 0; h0 < BN && seg.col0 + h0 < seg.width; h0 += d2) {
+					f32 kscale = seg.scale;
+					if (seg.heads) {   // L2NormMatrixWriter (gemm_b8.cuh:861-949): the tile holds BN / 2D whole heads
 						f32 ssum = 0.0f;
-						for (u32 c = 0; c < d; c += 32) {
+						for (u32 c = 0; c < p.head_dim; c += 32) {
 							u32 r[32];
 							tmem_ld_32x32b_x32(t_base + h0 + c, r);
 							tmem_wait_ld();
 #pragma unroll
 							for (u32 i = 0; i < 32; ++i) {
-								f32 f = acc_to_f32<F8>(r[i]);
+								f32 const f = acc_to_f32<F8>(r[i]);
 								ssum = __fmaf_rn(f, f, ssum);
 							}
 						}
-						f32 const kscale = __fmul_rn(rsqrt_approx(__fadd_rn(ssum, p.k0)), p.k1);
-						if (row_ok) p.rrms[u64(row) * p.rrms_cols + (col0 + h0) / (2 * d)] = kscale;
-						for (u32 c = 0; c < 2 * d; c += 32) {
-							u32 r[32];
-							tmem_ld_32x32b_x32(t_base + h0 + c, r);
-							tmem_wait_ld();
-							f32 const sc = c < d ? kscale : p.k2;
-							u32 w[8];
-#pragma unroll
-							for (u32 i = 0; i < 8; ++i) {
-								w[i] = pack4(u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 0]), sc))),
-											 u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 1]), sc))),
-											 u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 2]), sc))),
-											 u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 3]), sc))));
-							}
-							if (row_ok) {
-								uint4 *dst = reinterpret_cast<uint4 *>(
-									static_cast<i8 *>(p.c2) + u64(row) * p.c2_stride + col0 + h0 + c);
-								dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-								dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
-							}
-						}
+						kscale = __fmul_rn(rsqrt_approx(__fadd_rn(ssum, p.k0)), p.k1);
+						if (row_ok) p.rrms[u64(row) * p.rrms_cols + (seg.col0 + h0) / d2] = kscale;
 					}
-				}
-			} else if constexpr (EPI == EPI_L2NORM_KV) {
-				// raw columns of a head: [K(D) | V(D)]; the tile holds BN / 2D whole heads.
-				// k0 = eps, k1 = HEAD_SCALE (= out_scale * sqrt(D)), k2 = SEP_SCALE (= inp * out)
-				u32 const d = p.head_dim;
-				for (u32 h0 = 0; h0 < BN && n0 + h0 < p.n_raw; h0 += 2 * d) {
-					f32 ssum = 0.0f;
-					for (u32 c = 0; c < d; c += 32) {
-						u32 r[32];
+					for (u32 c = 0; c < d2; c += 32) {
+						u32 r[32], w[8];
 						tmem_ld_32x32b_x32(t_base + h0 + c, r);
 						tmem_wait_ld();
-#pragma unroll
-						for (u32 i = 0; i < 32; ++i) {
-							f32 f = acc_to_f32<F8>(r[i]);
-							ssum = __fmaf_rn(f, f, ssum);
-						}
-					}
-					f32 const kscale = __fmul_rn(rsqrt_approx(__fadd_rn(ssum, p.k0)), p.k1);
-					if (row_ok) {
-						p.rrms[u64(row) * p.rrms_cols + (n0 + h0) / (2 * d)] = kscale;
-					}
-					for (u32 c = 0; c < 2 * d; c += 32) {
-						u32 r[32];
-						tmem_ld_32x32b_x32(t_base + h0 + c, r);
-						tmem_wait_ld();
-						f32 const sc = c < d ? kscale : p.k2;
-						u32 w[8];
-#pragma unroll
-						for (u32 i = 0; i < 8; ++i) {
-							w[i] = pack4(
-								u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 0]), sc))),
-								u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 1]), sc))),
-								u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 2]), sc))),
-								u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 3]), sc))));
-						}
-						if (row_ok) {
-							uint4 *dst = reinterpret_cast<uint4 *>(
-								static_cast<i8 *>(p.c) + u64(row) * p.c_stride + n0 + h0 + c);
-							dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-							dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
-						}
+						scale32<F8>(r, seg.heads && c >= p.head_dim ? seg.scale : kscale, w);
+						if (row_ok) store32(seg.base + u64(row) * seg.stride + seg.col0 + h0 + c, w);
 					}
 				}
 			} else {
@@ -416,81 +417,7 @@ X17_DEV void gemm_body(CUtensorMap const *tm_a_ptr, CUtensorMap const *tm_b_ptr,
 					u32 r[32];
 					tmem_ld_32x32b_x32(t_base + c, r);
 					tmem_wait_ld();
-					if constexpr (EPI == EPI_SCALE_I8) {
-						// k0 = f32(inp_scale * out_scale)
-						u32 w[8];
-#pragma unroll
-						for (u32 i = 0; i < 8; ++i) {
-							w[i] = pack4(
-								u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 0]), p.k0))),
-								u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 1]), p.k0))),
-								u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 2]), p.k0))),
-								u32(f32_to_fixedi8(__fmul_rn(acc_to_f32<F8>(r[4 * i + 3]), p.k0))));
-						}
-						if (row_ok) {
-							uint4 *dst = reinterpret_cast<uint4 *>(
-								static_cast<i8 *>(p.c) + u64(row) * p.c_stride + n0 + c);
-							dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-							dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
-						}
-					} else if constexpr (EPI == EPI_RAW_I32) {
-						if (row_ok) {
-							uint4 *dst = reinterpret_cast<uint4 *>(
-								static_cast<u32 *>(p.c) + u64(row) * p.c_stride + n0 + c);
-#pragma unroll
-							for (u32 i = 0; i < 8; ++i) {
-								dst[i] = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
-							}
-						}
-					} else if constexpr (EPI == EPI_GEGLU_E4M3) {
-						u32 w[4];
-#pragma unroll
-						for (u32 i = 0; i < 4; ++i) {
-							u32 b[4];
-#pragma unroll
-							for (u32 j = 0; j < 4; ++j) {
-								f32 gate = acc_to_f32<F8>(r[8 * i + 2 * j]);
-								f32 lin = acc_to_f32<F8>(r[8 * i + 2 * j + 1]);
-								b[j] = f32_to_e4m3(geglu_val(gate, lin, p));
-							}
-							w[i] = pack4(b[0], b[1], b[2], b[3]);
-						}
-						if (row_ok) {
-							uint4 *dst = reinterpret_cast<uint4 *>(
-								static_cast<u8 *>(p.c) + u64(row) * p.c_stride + (n0 + c) / 2);
-							dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-						}
-					} else {  // EPI_RESID_E4M3 / EPI_RESID_I8
-						uint4 res = make_uint4(0, 0, 0, 0);
-						if (row_ok) {
-							res = *reinterpret_cast<uint4 const *>(
-								p.residual + u64(row) * p.resid_stride + (n0 + c) / 2);
-						}
-						u32 const rw[4] = {res.x, res.y, res.z, res.w};
-						u32 w[4];
-#pragma unroll
-						for (u32 i = 0; i < 4; ++i) {
-							u32 b[4];
-#pragma unroll
-							for (u32 j = 0; j < 4; ++j) {
-								f32 gate = acc_to_f32<F8>(r[8 * i + 2 * j]);
-								f32 val = acc_to_f32<F8>(r[8 * i + 2 * j + 1]);
-								i32 code = static_cast<i8>((rw[i] >> (8 * j)) & 0xFFu);
-								f32 v = resid_val(gate, val, f32(code), p);
-								if constexpr (EPI == EPI_RESID_E4M3) {
-									b[j] = f32_to_e4m3(v);
-								} else {
-									b[j] = u32(f32_to_fixedi8(v));
-								}
-							}
-							w[i] = pack4(b[0], b[1], b[2], b[3]);
-						}
-						if (row_ok) {
-							uint4 *dst = reinterpret_cast<uint4 *>(
-								static_cast<u8 *>(p.c) + u64(row) * p.c_stride + (n0 + c) / 2);
-							dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-						}
-					}
+					if (row_ok) store_cols32<EPI, F8>(r, p, row, n0 + c);
 				}
 			}
 			// this warp is done reading the accumulator buffer
@@ -512,6 +439,246 @@ X17_DEV void gemm_body(CUtensorMap const *tm_a_ptr, CUtensorMap const *tm_b_ptr,
 		tc_fence_after();
 		if constexpr (PAIR) tmem_dealloc_pair(tmem_base, 512);
 		else tmem_dealloc(tmem_base, 512);
+	}
+}
+
+// ---- few rows: K split over a cluster ------------------------------------------------------------
+//
+// With few rows of A a GEMM is a pass over the weights, and the persistent forms put at most one CTA on each column
+// tile: an 8192-column output keeps 32 of 148 SMs busy. Here a cluster of `split` CTAs shares one 128 x 256 tile, each
+// taking a contiguous part of K; the partial accumulators are exchanged through the cluster's shared memory (no
+// workspace, no second launch), the 32-column chunks of the tile being dealt out to the CTAs, which add the parts
+// up in K order and run the epilogue of their chunks. A's box is cut to the rows there are (the MMA reads 128 rows;
+// what lies behind the box only reaches accumulator rows that are never stored).
+// Bound by L2 -> SM traffic (weights once, A once per 256 columns; about 7.3 TB/s). Measured, weights cold, against
+// the one-CTA persistent form: 128 rows x [8192, 2 x 14336] e4m3 100 -> 48 us, 128 x [8192, 4096] int8 21 -> 17 us.
+struct SplitParams {
+	u32 split;     // CTAs per tile = cluster size: 1, 2 or 4
+	u32 a_rows;    // rows of A's box: a multiple of 8, at most 128
+	u32 stages;    // ring stages of a_rows * BK + B_BYTES
+	u32 tiles_m;
+	u32 slots;     // chunks of one other CTA that the ring has room for
+	// Which CTA of the cluster finishes chunk c of a tile (four bits per chunk), and how many of the chunks before c
+	// that CTA finishes too. [0]: plain tiles, dealt out in turn; [1]: tiles of whole heads [K(D) | V(D)], where the
+	// chunks of a K head stay together (one thread sums their squares in column order, as the other forms do) and the
+	// V chunks go to the CTAs behind.
+	u32 owner[2], before[2];
+};
+
+namespace gemm_cfg {
+constexpr u32 SPLIT_CHUNKS = BN / 32;
+constexpr u32 SPLIT_MAX = 4;
+constexpr u32 SPLIT_MAX_STAGES = 4;
+constexpr u32 split_smem_bytes(u32 a_rows, u32 stages) {
+	return stages * (a_rows * BK + B_BYTES) + 1024 /*alignment slack*/ + 256 /*barriers*/;
+}
+}  // namespace gemm_cfg
+
+template <int EPI, bool F8>
+__global__ void __launch_bounds__(gemm_cfg::THREADS, 2)
+gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const GemmParams p,
+				  const SplitParams sp) {
+	using namespace gemm_cfg;
+	constexpr bool HEADS = EPI == EPI_QKVG || EPI == EPI_L2NORM_KV;
+	constexpr u32 CHUNKS = SPLIT_CHUNKS;
+	extern __shared__ u8 smem_raw[];
+	u32 const smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+	u8 *const smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+	u32 const stage_bytes = sp.a_rows * BK + B_BYTES;
+	u32 const bar_base = smem_base + sp.stages * stage_bytes;
+	auto full_bar = [&](u32 s) { return bar_base + 8 * s; };
+	auto empty_bar = [&](u32 s) { return bar_base + 8 * (SPLIT_MAX_STAGES + s); };
+	u32 const acc_full_bar = bar_base + 8 * (2 * SPLIT_MAX_STAGES);
+	u32 const tmem_slot = acc_full_bar + 8;
+	volatile u32 *const tmem_slot_gen = reinterpret_cast<volatile u32 *>(smem_gen + (tmem_slot - smem_base));
+	volatile u32 *const abort_flag = tmem_slot_gen + 1;
+	WaitCtx const ctx{abort_flag, p.status};
+
+	u32 const warp = threadIdx.x >> 5;
+	u32 const lane = threadIdx.x & 31;
+	u32 const rank = cluster_cta_rank();
+	u32 const tile = blockIdx.x / sp.split;
+	u32 const m0 = (tile % sp.tiles_m) * BM;   // row tiles fastest: they read the same weights
+	u32 const n0 = (tile / sp.tiles_m) * BN;
+	u32 const k_blocks = p.k / BK;
+	u32 const kb_begin = rank * k_blocks / sp.split, kb_end = (rank + 1) * k_blocks / sp.split;
+
+	if (threadIdx.x == 0) {
+		for (u32 s = 0; s < sp.stages; ++s) {
+			mbar_init(full_bar(s), 1);
+			mbar_init(empty_bar(s), 1);
+		}
+		mbar_init(acc_full_bar, 1);
+		*abort_flag = 0;
+		mbar_fence_init();
+	}
+	if (warp == 1) {
+		tmem_alloc(tmem_slot, ACC_COLS);
+		tmem_relinquish();
+	}
+	tc_fence_before();
+	__syncthreads();
+	tc_fence_after();
+	u32 const tmem_base = *tmem_slot_gen;
+
+	bool ok = true;
+	if (warp == 0) {
+		if (elect_one()) {
+			tma_prefetch_desc(&tm_a);
+			tma_prefetch_desc(&tm_b);
+			for (u32 kb = kb_begin, s = 0, ph = 0; kb < kb_end; ++kb) {
+				if (!mbar_wait(empty_bar(s), ph ^ 1, ctx, ST_WAIT_STAGE_EMPTY, s)) break;
+				u32 const a_dst = smem_base + s * stage_bytes;
+				mbar_expect_tx(full_bar(s), stage_bytes);
+				tma_load_2d(a_dst + sp.a_rows * BK, &tm_b, full_bar(s), i32(kb * BK), i32(n0));
+				tma_load_2d(a_dst, &tm_a, full_bar(s), i32((kb * BK) % p.k_a), i32(m0));
+				if (++s == sp.stages) {
+					s = 0;
+					ph ^= 1;
+				}
+			}
+		}
+	} else if (warp == 1) {
+		if (elect_one()) {
+			constexpr u32 idesc = F8 ? make_idesc(DFMT_F32, FMT_E4M3, FMT_E4M3, 0, 0, BM, BN)
+									 : make_idesc(DFMT_S32, FMT_S8, FMT_S8, 0, 0, BM, BN);
+			bool done = true;
+			for (u32 kb = kb_begin, s = 0, ph = 0; kb < kb_end; ++kb) {
+				if (!mbar_wait(full_bar(s), ph, ctx, ST_WAIT_TMA_FULL, s)) {
+					done = false;
+					break;
+				}
+				tc_fence_after();
+				u32 const a_addr = smem_base + s * stage_bytes;
+				u64 const adesc = make_smem_desc(a_addr, 128);
+				u64 const bdesc = make_smem_desc(a_addr + sp.a_rows * BK, 128);
+#pragma unroll
+				for (u32 ks = 0; ks < BK / 32; ++ks) {
+					u32 const accumulate = kb != kb_begin || ks != 0 ? 1u : 0u;
+					if constexpr (F8) mma_f8_ss(tmem_base, adesc + 2 * ks, bdesc + 2 * ks, idesc, accumulate);
+					else mma_i8_ss(tmem_base, adesc + 2 * ks, bdesc + 2 * ks, idesc, accumulate);
+				}
+				tc_commit(empty_bar(s));
+				if (++s == sp.stages) {
+					s = 0;
+					ph ^= 1;
+				}
+			}
+			if (done) tc_commit(acc_full_bar);
+		}
+	} else {
+		ok = mbar_wait_warp(acc_full_bar, 0, ctx, ST_WAIT_ACC_FULL, 0);
+		tc_fence_after();
+	}
+	__syncwarp();
+
+	u32 const quarter = warp & 3;
+	u32 const row_in_tile = quarter * 32 + lane;
+	u32 const row = m0 + row_in_tile;
+	bool const row_ok = row < p.m;
+	bool const in_box = row_in_tile < sp.a_rows;
+	// uniform over the warp: an epilogue warp with rows to store
+	bool const works = warp >= 2 && ok && quarter * 32u < sp.a_rows && m0 + quarter * 32u < p.m;
+	u32 const t_base = tmem_base + ((quarter * 32u) << 16);
+	u32 const chunks = min(CHUNKS, (p.n_raw - n0) / 32);
+	u32 const chunk_bytes = sp.a_rows * 128;   // 8 x [a_rows][16 bytes]
+	u32 head_dim = 0;                          // of this tile, 0 where it holds plain columns
+	if constexpr (HEADS) head_dim = segment_of<EPI>(p, n0).heads ? p.head_dim : 0u;
+	// where chunk c of CTA `src` lands in the ring of the CTA that finishes it
+	u32 const owners = head_dim != 0 ? sp.owner[1] : sp.owner[0], befores = head_dim != 0 ? sp.before[1] : sp.before[0];
+	auto owner_of = [&](u32 c) { return (owners >> (4 * c)) & 15u; };
+	auto part_offset = [&](u32 c, u32 owner, u32 src) {
+		return ((src < owner ? src : src - 1) * sp.slots + ((befores >> (4 * c)) & 15u)) * chunk_bytes + row_in_tile * 16;
+	};
+	if (sp.split > 1) {
+		cluster_sync_all();   // every CTA's MMAs have finished: its ring takes the others' parts
+		if (works) {
+			for (u32 c = 0; c < chunks; ++c) {
+				u32 const owner = owner_of(c);
+				if (owner == rank) continue;
+				u32 r[32];
+				tmem_ld_32x32b_x32(t_base + 32 * c, r);
+				tmem_wait_ld();
+				u32 const dst = map_to_cta(smem_base + part_offset(c, owner, rank), owner);
+				if (in_box) {
+#pragma unroll
+					for (u32 g = 0; g < 8; ++g) {
+						st_cluster_v4(dst + g * sp.a_rows * 16, r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
+					}
+				}
+			}
+		}
+		cluster_sync_all();   // the parts have arrived
+	}
+	// chunk c of this row, added up over the cluster in K order
+	auto whole_chunk = [&](u32 c, u32 (&acc)[32]) {
+		u32 own[32];
+		tmem_ld_32x32b_x32(t_base + 32 * c, own);
+		tmem_wait_ld();
+#pragma unroll
+		for (u32 i = 0; i < 32; ++i) acc[i] = own[i];
+		if (sp.split > 1 && in_box) {
+#pragma unroll 1
+			for (u32 src = 0; src < sp.split; ++src) {
+				u32 const part = smem_base + part_offset(c, rank, src);   // (not read where src is this CTA)
+#pragma unroll
+				for (u32 g = 0; g < 8; ++g) {
+					uint4 v = make_uint4(own[4 * g], own[4 * g + 1], own[4 * g + 2], own[4 * g + 3]);
+					if (src != rank) v = ld_shared_v4(part + g * sp.a_rows * 16);
+					u32 const w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+					for (u32 i = 0; i < 4; ++i) {
+						u32 &a = acc[4 * g + i];
+						if (src == 0) a = w[i];
+						else if constexpr (F8) a = __float_as_uint(__fadd_rn(__uint_as_float(a), __uint_as_float(w[i])));
+						else a += w[i];
+					}
+				}
+			}
+		}
+	};
+	if (works) {
+		for (u32 c = 0; c < chunks; ++c) {
+			if (owner_of(c) != rank) continue;
+			u32 r[32];
+			if constexpr (HEADS) {
+				SegOut const seg = segment_of<EPI>(p, n0);
+				u32 last = c;
+				f32 sc = seg.scale;
+				if (head_dim != 0 && (32 * c) % (2 * head_dim) == 0) {   // a K head: its chunks follow one another
+					last = c + head_dim / 32 - 1;
+					f32 ssum = 0.0f;
+					for (u32 k = c; k <= last; ++k) {
+						whole_chunk(k, r);
+#pragma unroll
+						for (u32 i = 0; i < 32; ++i) {
+							f32 const f = acc_to_f32<F8>(r[i]);
+							ssum = __fmaf_rn(f, f, ssum);
+						}
+					}
+					sc = __fmul_rn(rsqrt_approx(__fadd_rn(ssum, p.k0)), p.k1);
+					if (row_ok) p.rrms[u64(row) * p.rrms_cols + (seg.col0 + 32 * c) / (2 * head_dim)] = sc;
+				}
+				for (; c <= last; ++c) {
+					u32 w[8];
+					whole_chunk(c, r);
+					scale32<F8>(r, sc, w);
+					if (row_ok) store32(seg.base + u64(row) * seg.stride + seg.col0 + 32 * c, w);
+				}
+				c = last;
+			} else {
+				whole_chunk(c, r);
+				if (row_ok) store_cols32<EPI, F8>(r, p, row, n0 + 32 * c);
+			}
+		}
+	}
+
+	tc_fence_before();
+	__syncthreads();
+	if (warp == 1) {
+		__syncwarp();
+		tc_fence_after();
+		tmem_dealloc(tmem_base, ACC_COLS);
 	}
 }
 

@@ -218,6 +218,16 @@ X17_DEV bool mbar_wait_warp(u32 bar, u32 parity, WaitCtx const &ctx, u32 code, u
 	return ok != 0;
 }
 
+X17_DEV uint4 ld_shared_v4(u32 addr) {
+	uint4 v;
+	asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+	return v;
+}
+X17_DEV void st_shared_v4(u32 addr, u32 a, u32 b, u32 c, u32 d) {
+	asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d)
+				 : "memory");
+}
+
 // generic-proxy writes to shared memory -> visible to the async proxy (TMA, tcgen05.mma)
 X17_DEV void fence_proxy_async_smem() {
 	asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -332,6 +342,11 @@ X17_DEV u32 map_to_cta(u32 smem_addr, u32 rank) {
 }
 X17_DEV void mbar_arrive_cluster(u32 bar_cluster) {
 	asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster) : "memory");
+}
+// 16 bytes into the shared memory of another CTA of the cluster (`addr_cluster`: an address from map_to_cta)
+X17_DEV void st_cluster_v4(u32 addr_cluster, u32 a, u32 b, u32 c, u32 d) {
+	asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr_cluster), "r"(a), "r"(b), "r"(c), "r"(d)
+				 : "memory");
 }
 X17_DEV void cluster_sync_all() {
 	asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");

@@ -73,12 +73,13 @@ def _dtype_and_device(op, name, t, dtype):
 ATTN_PERSISTENT, ATTN_PER_TILE = 0, 1
 
 
-GEMM_ONE_CTA, GEMM_CTA_PAIR = 0, 1
+GEMM_ONE_CTA, GEMM_CTA_PAIR, GEMM_AUTO = 0, 1, 2
 
 
-def set_gemm_tiling(tiling: int = GEMM_CTA_PAIR) -> None:
+def set_gemm_tiling(tiling: int = GEMM_AUTO) -> None:
     """Process-wide tiling of GemmKernel.launch and qkvg_fwd (x17ai_b200_set_gemm_tiling): clusters of two CTAs with
-    256 x 256 tiles (tcgen05.mma.cta_group::2, the default), or one CTA per SM with 128 x 256 tiles. Same bytes out."""
+    256 x 256 tiles (tcgen05.mma.cta_group::2), one CTA per SM with 128 x 256 tiles, or (default) chosen per launch
+    between the CTA pairs and, for few rows, K split over a cluster."""
     if _lib.load().x17ai_b200_set_gemm_tiling(int(tiling)) != 0:
         raise X17Error(f"unknown GEMM tiling {tiling}")
 
