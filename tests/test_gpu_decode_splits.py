@@ -1,0 +1,34 @@
+"""Split-KV decode at the edges of its forms: partials merged in a cluster's shared memory (up to 8 CTAs, then several
+splits per CTA), and through scratch memory above 64 splits; splits without keys; step counts of 0, 1 and more."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import code_hist
+from oracle import attn as o_attn
+from test_gpu_decode import _case
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("D,kv_len,W,splits", [(128, 700, 0, 2), (64, 1024, 0, 8), (128, 1024, 0, 9), (32, 2048, 0, 16),
+                                               (128, 2048, 0, 17), (64, 2048, 1024, 40), (128, 2048, 0, 64), (128, 2048, 0, 65),
+                                               (128, 100, 0, 16), (128, 1, 0, 3), (128, 2048, 0, 0)])
+def test_decode_split_forms(stream, D, kv_len, W, splits):
+    from x17ai_b200 import kernels as K
+    B, H, T = 2, 3, 2048
+    rng = np.random.default_rng(D + kv_len + splits)
+    q, kv, sk, sv, temp = _case(rng, B, H, D, T)
+    kern = K.AttnKernel(K.AttnKernelConfig(H, D, H * D, 2 * H * D, H * D))
+    dev = [torch.from_numpy(a).cuda() for a in (q, kv, sk, sv, temp)]
+    ref_out, ref_l = o_attn.attn_decode_i8(q, kv, kv_len, sk, sv, temp, W, H, D, kv_tile=1 << 20)
+    for no_alloc in (False, True):
+        out = torch.zeros((B, H * D), dtype=torch.int8, device="cuda")
+        l = torch.zeros((B, H), dtype=torch.float32, device="cuda")
+        torch.cuda.synchronize()
+        kern.decode(stream, dev[0], dev[1], kv_len, dev[2], dev[3], dev[4], out, l, window_size=W, n_splits=splits, no_alloc=no_alloc)
+        stream.synchronize()
+        hist = code_hist(out.cpu().numpy(), ref_out)
+        # P is rounded against running maxima here, against the final one in the oracle: at most one code apart
+        assert hist[2:].sum() == 0 and hist[1] / ref_out.size <= 0.08, hist
+        assert np.max(np.abs(l.cpu().numpy() - ref_l)) <= 1e-3

@@ -679,6 +679,99 @@ __global__ void split_i8_weights_kernel(int8_t const *w, uint64_t rows, uint64_t
 
 
 
+// ---- decode ------------------------------------------------------------------------------------
+
+// Checks and parameters shared by the two decode entry points.
+x17ai_DiagnosticBuffer *check_decode(char const *who, x17ai_AttnConfig const *cfg, size_t batch, int8_t const *q,
+									 int8_t const *kv_cache, size_t kv_capacity, size_t kv_len, int8_t const *sink_k,
+									 int8_t const *sink_v, float const *attn_temperature, int8_t const *out, size_t window_size) {
+	if (auto *d = check_attn_config(cfg, who)) return d;
+	if (batch == 0) return make_diag("x17ai_b200: empty decode input", who, ": decode input q has zero size");
+	if (batch > 65535 || kv_capacity >= (size_t(1) << 31) || kv_len > kv_capacity) {
+		return make_diag("x17ai_b200: decode shape out of range", who, ": decode shape out of range (kv_len ",
+						 kv_len, ", kv_capacity ", kv_capacity, ")");
+	}
+	if (window_size > 0 && window_size % 16 != 0) {
+		return make_diag("x17ai_b200: bad window", who,
+						 ": attention window_size must be zero or divisible by 16, got ", window_size);
+	}
+	if (!q || !kv_cache || !sink_k || !sink_v || !attn_temperature || !out) {
+		return make_diag("x17ai_b200: null tensor", who, ": null tensor argument");
+	}
+	if (!aligned16(q) || !aligned16(kv_cache) || !aligned16(sink_k)) {
+		return make_diag("x17ai_b200: misaligned tensor", who, ": tensors must be 16-byte aligned");
+	}
+	return nullptr;
+}
+
+// Enough CTAs for two waves of 4 CTAs per SM, no split shorter than 256 keys.
+size_t choose_splits(size_t pairs, size_t kv_len, int sm_count) {
+	size_t const want = size_t(sm_count) * 8;
+	size_t n = pairs >= want ? 1 : (want + pairs - 1) / pairs;
+	size_t const most = kv_len / 256 > 0 ? kv_len / 256 : 1;
+	return n > most ? most : n;
+}
+
+x17::DecodeParams decode_params(x17ai_AttnConfig const *cfg, int8_t const *q, int8_t const *kv_cache, size_t kv_capacity,
+								size_t kv_len, uint32_t const *kv_lens, int8_t const *sink_k, int8_t const *sink_v,
+								float const *attn_temperature, int8_t *out, float *l, size_t window_size, size_t n_splits) {
+	x17::DecodeParams p{};
+	p.q = q;
+	p.q_stride = cfg->q_stride;
+	p.kv = kv_cache;
+	p.kv_stride = cfg->kv_stride;
+	p.kv_batch_stride = cfg->kv_stride * kv_capacity;
+	p.kv_lens = kv_lens;
+	p.kv_len = uint32_t(kv_len);
+	p.kv_capacity = uint32_t(kv_capacity);
+	p.window = window_size == 0 ? 0xFFFFFFFFu : uint32_t(((window_size - 1) / 16 + 1) * 16);
+	p.sink_k = sink_k;
+	p.sink_v = sink_v;
+	p.temperature = attn_temperature;
+	p.out = out;
+	p.o_stride = cfg->o_stride;
+	p.l = l;
+	p.n_heads = uint32_t(cfg->n_heads);
+	p.n_splits = uint32_t(n_splits);
+	return p;
+}
+
+// Splits whose partials meet in a cluster's shared memory (the others need p.scratch).
+bool decode_in_cluster(size_t n_splits) { return n_splits <= x17::dec_cfg::MAX_CLUSTER_SPLITS; }
+
+template <uint32_t D>
+x17ai_DiagnosticBuffer *decode_go_dim(char const *who, cudaStream_t s, size_t batch, x17::DecodeParams const &p) {
+	using namespace x17::dec_cfg;
+	if (p.n_splits > 1 && p.scratch == nullptr) {
+		auto const kernel = x17::attn_decode_kernel<D>;
+		uint32_t const z = p.n_splits < MAX_CLUSTER ? p.n_splits : MAX_CLUSTER;
+		cudaLaunchAttribute attr{};
+		attr.id = cudaLaunchAttributeClusterDimension;
+		attr.val.clusterDim.x = 1;
+		attr.val.clusterDim.y = 1;
+		attr.val.clusterDim.z = z;
+		cudaLaunchConfig_t cfg{};
+		cfg.gridDim = dim3(p.n_heads, unsigned(batch), z);
+		cfg.blockDim = dim3(THREADS);
+		cfg.dynamicSmemBytes = partials_bytes<D>(p.n_splits);
+		cfg.stream = s;
+		cfg.attrs = &attr;
+		cfg.numAttrs = 1;
+		cudaLaunchKernelEx(&cfg, kernel, p);   // launch_result() reads the error
+		return launch_result(who);
+	}
+	x17::attn_decode_kernel<D><<<dim3(p.n_heads, unsigned(batch), p.n_splits), THREADS, 0, s>>>(p);
+	if (p.n_splits > 1) x17::attn_decode_merge_kernel<D><<<dim3(p.n_heads, unsigned(batch)), D, 0, s>>>(p);
+	x17ai_DiagnosticBuffer *res = launch_result(who);
+	if (res == nullptr && p.n_splits > 1) g_launches.fetch_add(1, std::memory_order_relaxed);
+	return res;
+}
+x17ai_DiagnosticBuffer *decode_go(char const *who, cudaStream_t s, size_t head_dim, size_t batch, x17::DecodeParams const &p) {
+	return head_dim == 128 ? decode_go_dim<128>(who, s, batch, p)
+		   : head_dim == 64 ? decode_go_dim<64>(who, s, batch, p)
+							: decode_go_dim<32>(who, s, batch, p);
+}
+
 // ---- decode without allocation -------------------------------------------------------------------
 // Scratch for the split-KV partials of x17ai_b200_attn_decode_i8_noalloc. It lives in the
 // library image: every GPU that loads the library holds these 4 MiB until the process exits.
@@ -1041,80 +1134,28 @@ x17ai_DiagnosticBuffer *x17ai_b200_attn_decode_i8(
 	uint32_t const *kv_lens, int8_t const *sink_k, int8_t const *sink_v,
 	float const *attn_temperature, int8_t *out, float *l, size_t window_size, size_t n_splits) {
 	char const *who = "x17ai_b200_attn_decode_i8()";
-	if (auto *d = check_attn_config(cfg, who)) return d;
-	if (batch == 0) return make_diag("x17ai_b200: empty decode input", who, ": decode input q has zero size");
-	if (batch > 65535 || kv_capacity >= (size_t(1) << 31) || kv_len > kv_capacity) {
-		return make_diag("x17ai_b200: decode shape out of range", who, ": decode shape out of range (kv_len ",
-						 kv_len, ", kv_capacity ", kv_capacity, ")");
-	}
-	if (window_size > 0 && window_size % 16 != 0) {
-		return make_diag("x17ai_b200: bad window", who,
-						 ": attention window_size must be zero or divisible by 16, got ", window_size);
-	}
-	if (!q || !kv_cache || !sink_k || !sink_v || !attn_temperature || !out) {
-		return make_diag("x17ai_b200: null tensor", who, ": null tensor argument");
-	}
-	if (!aligned16(q) || !aligned16(kv_cache) || !aligned16(sink_k)) {
-		return make_diag("x17ai_b200: misaligned tensor", who, ": tensors must be 16-byte aligned");
+	if (auto *d = check_decode(who, cfg, batch, q, kv_cache, kv_capacity, kv_len, sink_k, sink_v, attn_temperature, out,
+							   window_size)) {
+		return d;
 	}
 	StreamScope scope(stream, who);
 	if (scope.diag) return scope.diag;
 	cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-
 	size_t const pairs = batch * cfg->n_heads;
-	if (n_splits == 0) {  // choose: enough CTAs for two waves of 4 CTAs per SM
-		size_t const want = size_t(scope.state().sm_count) * 8;
-		n_splits = pairs >= want ? 1 : (want + pairs - 1) / pairs;
-		size_t const max_splits = kv_len / 256 > 0 ? kv_len / 256 : 1;
-		if (n_splits > max_splits) n_splits = max_splits;
-	}
+	if (n_splits == 0) n_splits = choose_splits(pairs, kv_len, scope.state().sm_count);
 	if (n_splits > 65535) n_splits = 65535;
-
-	uint32_t const d = uint32_t(cfg->head_dim);
-	x17::DecodeParams p{};
-	p.q = q;
-	p.q_stride = cfg->q_stride;
-	p.kv = kv_cache;
-	p.kv_stride = cfg->kv_stride;
-	p.kv_batch_stride = cfg->kv_stride * kv_capacity;
-	p.kv_lens = kv_lens;
-	p.kv_len = uint32_t(kv_len);
-	p.kv_capacity = uint32_t(kv_capacity);
-	p.window = window_size == 0 ? 0xFFFFFFFFu : uint32_t(((window_size - 1) / 16 + 1) * 16);
-	p.sink_k = sink_k;
-	p.sink_v = sink_v;
-	p.temperature = attn_temperature;
-	p.out = out;
-	p.o_stride = cfg->o_stride;
-	p.l = l;
-	p.n_heads = uint32_t(cfg->n_heads);
-	p.n_splits = uint32_t(n_splits);
-	p.scratch = nullptr;
-	if (n_splits > 1) {
-		size_t const bytes = pairs * n_splits * (d + 2) * sizeof(float);
+	x17::DecodeParams p = decode_params(cfg, q, kv_cache, kv_capacity, kv_len, kv_lens, sink_k, sink_v, attn_temperature, out,
+										l, window_size, n_splits);
+	if (!decode_in_cluster(n_splits)) {
+		size_t const bytes = pairs * n_splits * (cfg->head_dim + 2) * sizeof(float);
 		cudaError_t e = cudaMallocAsync(reinterpret_cast<void **>(&p.scratch), bytes, s);
 		if (e != cudaSuccess) {
 			return make_diag("x17ai_b200: scratch allocation failed", who, ": cudaMallocAsync(", bytes,
 							 ") failed: ", cudaGetErrorString(e));
 		}
 	}
-	dim3 grid(unsigned(cfg->n_heads), unsigned(batch), unsigned(n_splits));
-	dim3 mgrid(unsigned(cfg->n_heads), unsigned(batch));
-	if (d == 128) {
-		x17::attn_decode_kernel<128><<<grid, x17::dec_cfg::THREADS, 0, s>>>(p);
-		if (n_splits > 1) x17::attn_decode_merge_kernel<128><<<mgrid, 128, 0, s>>>(p);
-	} else if (d == 64) {
-		x17::attn_decode_kernel<64><<<grid, x17::dec_cfg::THREADS, 0, s>>>(p);
-		if (n_splits > 1) x17::attn_decode_merge_kernel<64><<<mgrid, 64, 0, s>>>(p);
-	} else {
-		x17::attn_decode_kernel<32><<<grid, x17::dec_cfg::THREADS, 0, s>>>(p);
-		if (n_splits > 1) x17::attn_decode_merge_kernel<32><<<mgrid, 32, 0, s>>>(p);
-	}
-	x17ai_DiagnosticBuffer *res = launch_result(who);
-	if (n_splits > 1) {
-		if (res == nullptr) g_launches.fetch_add(1, std::memory_order_relaxed);
-		cudaFreeAsync(p.scratch, s);
-	}
+	x17ai_DiagnosticBuffer *res = decode_go(who, s, cfg->head_dim, batch, p);
+	if (p.scratch != nullptr) cudaFreeAsync(p.scratch, s);
 	return res;
 }
 
@@ -1124,21 +1165,9 @@ x17ai_DiagnosticBuffer *x17ai_b200_attn_decode_i8_noalloc(
 	uint32_t const *kv_lens, int8_t const *sink_k, int8_t const *sink_v,
 	float const *attn_temperature, int8_t *out, float *l, size_t window_size, size_t n_splits) {
 	char const *who = "x17ai_b200_attn_decode_i8_noalloc()";
-	if (auto *d = check_attn_config(cfg, who)) return d;
-	if (batch == 0) return make_diag("x17ai_b200: empty decode input", who, ": decode input q has zero size");
-	if (batch > 65535 || kv_capacity >= (size_t(1) << 31) || kv_len > kv_capacity) {
-		return make_diag("x17ai_b200: decode shape out of range", who, ": decode shape out of range (kv_len ",
-						 kv_len, ", kv_capacity ", kv_capacity, ")");
-	}
-	if (window_size > 0 && window_size % 16 != 0) {
-		return make_diag("x17ai_b200: bad window", who,
-						 ": attention window_size must be zero or divisible by 16, got ", window_size);
-	}
-	if (!q || !kv_cache || !sink_k || !sink_v || !attn_temperature || !out) {
-		return make_diag("x17ai_b200: null tensor", who, ": null tensor argument");
-	}
-	if (!aligned16(q) || !aligned16(kv_cache) || !aligned16(sink_k)) {
-		return make_diag("x17ai_b200: misaligned tensor", who, ": tensors must be 16-byte aligned");
+	if (auto *d = check_decode(who, cfg, batch, q, kv_cache, kv_capacity, kv_len, sink_k, sink_v, attn_temperature, out,
+							   window_size)) {
+		return d;
 	}
 	if (stream == nullptr) return make_diag("x17ai_b200: null stream", who, ": null stream");
 	if (!x17::driver().ok) {
@@ -1193,12 +1222,7 @@ x17ai_DiagnosticBuffer *x17ai_b200_attn_decode_i8_noalloc(
 	}
 	cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
 	size_t const pairs = batch * cfg->n_heads;
-	if (n_splits == 0) {
-		size_t const want = size_t(nd.sm_count) * 8;
-		n_splits = pairs >= want ? 1 : (want + pairs - 1) / pairs;
-		size_t const max_splits = kv_len / 256 > 0 ? kv_len / 256 : 1;
-		if (n_splits > max_splits) n_splits = max_splits;
-	}
+	if (n_splits == 0) n_splits = choose_splits(pairs, kv_len, nd.sm_count);
 	uint32_t const d = uint32_t(cfg->head_dim);
 	size_t const need = n_splits > 1 ? pairs * n_splits * (d + 2) : 0;
 	if (n_splits > 65535 || need > NOALLOC_SCRATCH_FLOATS) {
@@ -1206,40 +1230,10 @@ x17ai_DiagnosticBuffer *x17ai_b200_attn_decode_i8_noalloc(
 						 need, " floats exceeds the built-in scratch of ", NOALLOC_SCRATCH_FLOATS,
 						 " floats (4 MiB); use fewer splits or x17ai_b200_attn_decode_i8");
 	}
-	x17::DecodeParams p{};
-	p.q = q;
-	p.q_stride = cfg->q_stride;
-	p.kv = kv_cache;
-	p.kv_stride = cfg->kv_stride;
-	p.kv_batch_stride = cfg->kv_stride * kv_capacity;
-	p.kv_lens = kv_lens;
-	p.kv_len = uint32_t(kv_len);
-	p.kv_capacity = uint32_t(kv_capacity);
-	p.window = window_size == 0 ? 0xFFFFFFFFu : uint32_t(((window_size - 1) / 16 + 1) * 16);
-	p.sink_k = sink_k;
-	p.sink_v = sink_v;
-	p.temperature = attn_temperature;
-	p.out = out;
-	p.o_stride = cfg->o_stride;
-	p.l = l;
-	p.n_heads = uint32_t(cfg->n_heads);
-	p.n_splits = uint32_t(n_splits);
-	p.scratch = nd.scratch;  // every split writes its whole slot before the merge reads it
-	dim3 grid(unsigned(cfg->n_heads), unsigned(batch), unsigned(n_splits));
-	dim3 mgrid(unsigned(cfg->n_heads), unsigned(batch));
-	if (d == 128) {
-		x17::attn_decode_kernel<128><<<grid, x17::dec_cfg::THREADS, 0, s>>>(p);
-		if (n_splits > 1) x17::attn_decode_merge_kernel<128><<<mgrid, 128, 0, s>>>(p);
-	} else if (d == 64) {
-		x17::attn_decode_kernel<64><<<grid, x17::dec_cfg::THREADS, 0, s>>>(p);
-		if (n_splits > 1) x17::attn_decode_merge_kernel<64><<<mgrid, 64, 0, s>>>(p);
-	} else {
-		x17::attn_decode_kernel<32><<<grid, x17::dec_cfg::THREADS, 0, s>>>(p);
-		if (n_splits > 1) x17::attn_decode_merge_kernel<32><<<mgrid, 32, 0, s>>>(p);
-	}
-	x17ai_DiagnosticBuffer *res = launch_result(who);
-	if (res == nullptr && n_splits > 1) g_launches.fetch_add(1, std::memory_order_relaxed);
-	return res;
+	x17::DecodeParams p = decode_params(cfg, q, kv_cache, kv_capacity, kv_len, kv_lens, sink_k, sink_v, attn_temperature, out,
+										l, window_size, n_splits);
+	if (!decode_in_cluster(n_splits)) p.scratch = nd.scratch;  // every split writes its whole slot before the merge reads it
+	return decode_go(who, s, cfg->head_dim, batch, p);
 }
 
 x17ai_DiagnosticBuffer *x17ai_b200_gemm_meta(x17ai_GemmConfig const *cfg, x17ai_GemmMeta *meta) {

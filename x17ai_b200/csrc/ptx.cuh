@@ -348,6 +348,15 @@ X17_DEV void st_cluster_v4(u32 addr_cluster, u32 a, u32 b, u32 c, u32 d) {
 	asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr_cluster), "r"(a), "r"(b), "r"(c), "r"(d)
 				 : "memory");
 }
+X17_DEV void st_cluster_f32(u32 addr_cluster, f32 v) {
+	asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr_cluster), "f"(v) : "memory");
+}
+X17_DEV void cluster_arrive() {
+	asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+X17_DEV void cluster_wait() {
+	asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 X17_DEV void cluster_sync_all() {
 	asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
