@@ -160,6 +160,24 @@ def load():
     return lib
 
 
+_hostcall = None
+
+
+def hostcall():
+    """The native launch path (csrc/hostcall.cpp), bound to the loaded library's entry points."""
+    global _hostcall
+    if _hostcall is None:
+        lib = load()
+        try:
+            import torch  # noqa: F401  (its libraries have to be loaded first)
+            from . import _hostcall as mod
+        except ImportError as e:
+            raise X17Error(f"x17ai_b200/_hostcall.so is missing or does not load ({e}): build it with `python -m x17ai_b200.build`")
+        mod.init({name: ctypes.cast(getattr(lib, name), c_void_p).value for name in mod.entries()})
+        _hostcall = mod
+    return _hostcall
+
+
 def take_diag(diag) -> str:
     lib = load()
     buf = ctypes.create_string_buffer(4096)

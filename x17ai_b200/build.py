@@ -1,5 +1,5 @@
-"""Builds libx17ai_b200.so in-tree with nvcc for sm_100a (no JIT cache: the built library
-travels with the source tree)."""
+"""Builds libx17ai_b200.so in-tree with nvcc for sm_100a, and the native launch path _hostcall.so with the host
+compiler (no JIT cache: the built libraries travel with the source tree)."""
 import os
 import subprocess
 import sys
@@ -8,6 +8,7 @@ from pathlib import Path
 HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 LIB = HERE / "libx17ai_b200.so"
+HOSTCALL = HERE / "_hostcall.so"
 SOURCES = [CSRC / "api.cu", CSRC / "shim.cpp"]
 HEADERS = sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.hpp")) + [HERE.parent / "include" / "x17ai_b200.h"]
 
@@ -28,6 +29,7 @@ def needs_build() -> bool:
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
+    build_hostcall(force)
     if os.environ.get("X17AI_B200_LIB"):
         return Path(os.environ["X17AI_B200_LIB"])
     if not force and not needs_build():
@@ -43,6 +45,25 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     if verbose:
         print(log)
     return LIB
+
+
+def build_hostcall(force: bool = False) -> Path:
+    """The native launch path (csrc/hostcall.cpp), a CPython extension over torch's headers."""
+    src = CSRC / "hostcall.cpp"
+    deps = (src, HERE.parent / "include" / "x17ai_b200.h")
+    if not force and HOSTCALL.exists() and all(d.stat().st_mtime <= HOSTCALL.stat().st_mtime for d in deps):
+        return HOSTCALL
+    import sysconfig
+    import torch
+    t = Path(torch.__path__[0])
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-I{t}/include", f"-I{t}/include/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}",
+           str(src), "-o", str(HOSTCALL), f"-L{t}/lib", "-ltorch_python", "-ltorch_cpu", "-lc10"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError("g++ failed building _hostcall.so")
+    return HOSTCALL
 
 
 def build_kernel_objects():

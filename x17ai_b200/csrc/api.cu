@@ -66,13 +66,17 @@ struct StreamScope {
 			return;
 		}
 		CUresult e = DRV(cuStreamGetCtx)(reinterpret_cast<CUstream>(stream), &ctx);
-		if (e == CUDA_SUCCESS) e = DRV(cuCtxPushCurrent)(ctx);
+		CUcontext current = nullptr;
+		if (e == CUDA_SUCCESS) e = DRV(cuCtxGetCurrent)(&current);
+		if (e == CUDA_SUCCESS && current != ctx) {   // (a program that also runs torch has it current already)
+			e = DRV(cuCtxPushCurrent)(ctx);
+			pushed = e == CUDA_SUCCESS;
+		}
 		if (e != CUDA_SUCCESS) {
 			diag = make_diag("x17ai_b200: cannot enter the stream's context", who,
 							 ": cannot enter the stream's context: ", x17::cu_error_text(e));
 			return;
 		}
-		pushed = true;
 		CUdevice dev;
 		e = DRV(cuCtxGetDevice)(&dev);
 		if (e != CUDA_SUCCESS || int(dev) < 0 || int(dev) >= MAX_DEVICES) {
@@ -107,6 +111,20 @@ struct StreamScope {
 	}
 	DeviceState &state() const { return g_dev[device]; }
 };
+
+// Raises a kernel's dynamic shared memory limit, once per kernel and device.
+template <auto KERNEL>
+struct Kernel {};
+template <auto KERNEL>
+cudaError_t allow_smem(Kernel<KERNEL>, int device, uint32_t bytes) {
+	static_assert(MAX_DEVICES <= 32);
+	static std::atomic<uint32_t> done{0};
+	uint32_t const bit = 1u << device;
+	if ((done.load(std::memory_order_acquire) & bit) != 0) return cudaSuccess;
+	cudaError_t const e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
+	if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+	return e;
+}
 
 x17ai_DiagnosticBuffer *launch_result(char const *who) {
 	cudaError_t e = cudaGetLastError();
@@ -290,38 +308,32 @@ x17ai_DiagnosticBuffer *attn_launch(
 		plan.n_items = uint32_t(items);
 		dim3 grid(plan.n_items < sms ? plan.n_items : sms);
 		dim3 block(x17::attn_stream_cfg::THREADS);
-		auto go = [&](auto kernel, uint32_t smem) -> cudaError_t {
-			cudaError_t e2 = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+		auto go = [&](auto tag, auto kernel, uint32_t smem) -> cudaError_t {
+			cudaError_t e2 = allow_smem(tag, scope.device, smem);
 			if (e2 != cudaSuccess) return e2;
 			kernel<<<grid, block, smem, reinterpret_cast<cudaStream_t>(stream)>>>(tm_q, tm_kv, p, plan);
 			return cudaSuccess;
 		};
-		if (d == 128) {
-			ce = go(x17::attn_fwd_stream_kernel<128, DEBUG, FP8PV>, x17::attn_stream_cfg::smem_bytes<128>());
-		} else if (d == 64) {
-			ce = go(x17::attn_fwd_stream_kernel<64, DEBUG, FP8PV>, x17::attn_stream_cfg::smem_bytes<64>());
-		} else {
-			ce = go(x17::attn_fwd_stream_kernel<32, DEBUG, FP8PV>, x17::attn_stream_cfg::smem_bytes<32>());
-		}
+#define X17_GO(DIM) go(Kernel<&x17::attn_fwd_stream_kernel<DIM, DEBUG, FP8PV>>{}, x17::attn_fwd_stream_kernel<DIM, DEBUG, FP8PV>, \
+					   x17::attn_stream_cfg::smem_bytes<DIM>())
+		ce = d == 128 ? X17_GO(128) : d == 64 ? X17_GO(64) : X17_GO(32);
+#undef X17_GO
 	} else {
 		dim3 grid(unsigned((seq_len + x17::attn_cfg::BQ - 1) / x17::attn_cfg::BQ), unsigned(cfg->n_heads),
 				  unsigned(batch));
 		dim3 block(x17::attn_cfg::THREADS);
-		auto go = [&](auto kernel, uint32_t smem) -> cudaError_t {
+		auto go = [&](auto tag, auto kernel, uint32_t smem) -> cudaError_t {
 			// at least 80 KB so that no more than two CTAs (2 x 256 TMEM columns) share an SM
 			smem = smem < 80u * 1024u ? 80u * 1024u : smem;
-			cudaError_t e2 = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+			cudaError_t e2 = allow_smem(tag, scope.device, smem);
 			if (e2 != cudaSuccess) return e2;
 			kernel<<<grid, block, smem, reinterpret_cast<cudaStream_t>(stream)>>>(tm_q, tm_kv, p);
 			return cudaSuccess;
 		};
-		if (d == 128) {
-			ce = go(x17::attn_fwd_kernel<128, DEBUG, FP8PV, SCALED>, x17::attn_cfg::smem_bytes<128>());
-		} else if (d == 64) {
-			ce = go(x17::attn_fwd_kernel<64, DEBUG, FP8PV, SCALED>, x17::attn_cfg::smem_bytes<64>());
-		} else {
-			ce = go(x17::attn_fwd_kernel<32, DEBUG, FP8PV, SCALED>, x17::attn_cfg::smem_bytes<32>());
-		}
+#define X17_GO(DIM) go(Kernel<&x17::attn_fwd_kernel<DIM, DEBUG, FP8PV, SCALED>>{}, x17::attn_fwd_kernel<DIM, DEBUG, FP8PV, SCALED>, \
+					   x17::attn_cfg::smem_bytes<DIM>())
+		ce = d == 128 ? X17_GO(128) : d == 64 ? X17_GO(64) : X17_GO(32);
+#undef X17_GO
 	}
 	if (ce != cudaSuccess) {
 		return make_diag("x17ai_b200: cudaFuncSetAttribute failed", who, ": cudaFuncSetAttribute failed: ",
@@ -476,23 +488,23 @@ uint32_t max_pair_clusters(Kernel kernel, uint32_t smem, int sm_count) {
 // The CTA-pair form (gemm.cuh): clusters of two CTAs, one 256 x 256 tile per cluster. `tb_half` is B's map with a box
 // of half a tile's rows. Used for more than one row tile unless the tiling is X17AI_B200_GEMM_ONE_CTA.
 template <int EPI, bool F8>
-cudaError_t gemm_go_pair_kind(int sm_count, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tb_half,
+cudaError_t gemm_go_pair_kind(StreamScope const &on, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tb_half,
 							  x17::GemmParams const &p) {
 	uint32_t const smem = x17::gemm_cfg::PAIR_SMEM_BYTES;
 	auto const kernel = x17::gemm_pair_kernel<EPI, F8>;
-	cudaError_t const ce = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+	cudaError_t const ce = allow_smem(Kernel<&x17::gemm_pair_kernel<EPI, F8>>{}, on.device, smem);
 	if (ce != cudaSuccess) return ce;
 	uint32_t const tiles = ((p.m + 2 * x17::gemm_cfg::BM - 1) / (2 * x17::gemm_cfg::BM)) * p.tiles_n;
-	uint32_t const fit = max_pair_clusters(kernel, smem, sm_count);
+	uint32_t const fit = max_pair_clusters(kernel, smem, on.state().sm_count);
 	uint32_t const clusters = tiles < fit ? tiles : fit;
 	kernel<<<dim3(2 * clusters), x17::gemm_cfg::THREADS, smem, stream>>>(ta, tb_half, p);
 	return cudaSuccess;
 }
 template <int EPI>
-cudaError_t gemm_go_pair(bool f8, int sm_count, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tb_half,
+cudaError_t gemm_go_pair(bool f8, StreamScope const &on, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tb_half,
 						 x17::GemmParams const &p) {
-	return f8 ? gemm_go_pair_kind<EPI, true>(sm_count, stream, ta, tb_half, p)
-			  : gemm_go_pair_kind<EPI, false>(sm_count, stream, ta, tb_half, p);
+	return f8 ? gemm_go_pair_kind<EPI, true>(on, stream, ta, tb_half, p)
+			  : gemm_go_pair_kind<EPI, false>(on, stream, ta, tb_half, p);
 }
 
 // The form for few rows (gemm.cuh): a cluster of up to four CTAs shares one 128 x 256 tile, K split over it.
@@ -555,12 +567,11 @@ SplitPlan plan_split(size_t rows, size_t n_raw, size_t k, uint32_t head_dim, int
 }
 
 template <int EPI, bool F8>
-cudaError_t gemm_go_split_kind(SplitPlan const &plan, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tb,
+cudaError_t gemm_go_split_kind(StreamScope const &on, SplitPlan const &plan, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tb,
 							   x17::GemmParams const &p) {
 	auto const kernel = x17::gemm_split_kernel<EPI, F8>;
 	using namespace x17::gemm_cfg;
-	cudaError_t const ce = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-												int(split_smem_bytes(BM, SPLIT_MAX_STAGES)));
+	cudaError_t const ce = allow_smem(Kernel<&x17::gemm_split_kernel<EPI, F8>>{}, on.device, split_smem_bytes(BM, SPLIT_MAX_STAGES));
 	if (ce != cudaSuccess) return ce;
 	cudaLaunchAttribute attr{};
 	attr.id = cudaLaunchAttributeClusterDimension;
@@ -577,9 +588,9 @@ cudaError_t gemm_go_split_kind(SplitPlan const &plan, cudaStream_t stream, CUten
 	return cudaLaunchKernelEx(&cfg, kernel, ta, tb, p, plan.sp);
 }
 template <int EPI>
-cudaError_t gemm_go_split(bool f8, SplitPlan const &plan, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tb,
+cudaError_t gemm_go_split(bool f8, StreamScope const &on, SplitPlan const &plan, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tb,
 						  x17::GemmParams const &p) {
-	return f8 ? gemm_go_split_kind<EPI, true>(plan, stream, ta, tb, p) : gemm_go_split_kind<EPI, false>(plan, stream, ta, tb, p);
+	return f8 ? gemm_go_split_kind<EPI, true>(on, plan, stream, ta, tb, p) : gemm_go_split_kind<EPI, false>(on, plan, stream, ta, tb, p);
 }
 
 // The form for up to 48 rows (gemm_rows.cuh; above that its L2 -> SM traffic, the tokens' bytes once per 128 columns,
@@ -614,10 +625,10 @@ RowsPlan plan_rows(size_t rows, size_t n_raw, size_t k, bool heads, int sm_count
 }
 
 template <int EPI, bool F8>
-cudaError_t gemm_go_rows_kind(RowsPlan const &plan, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tw,
+cudaError_t gemm_go_rows_kind(StreamScope const &on, RowsPlan const &plan, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tw,
 							  x17::GemmParams const &p) {
 	auto const kernel = x17::gemm_rows_kernel<EPI, F8>;
-	cudaError_t const ce = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
+	cudaError_t const ce = allow_smem(Kernel<&x17::gemm_rows_kernel<EPI, F8>>{}, on.device, 112 * 1024);
 	if (ce != cudaSuccess) return ce;
 	cudaLaunchAttribute attr{};
 	attr.id = cudaLaunchAttributeClusterDimension;
@@ -634,26 +645,24 @@ cudaError_t gemm_go_rows_kind(RowsPlan const &plan, cudaStream_t stream, CUtenso
 	return cudaLaunchKernelEx(&cfg, kernel, ta, tw, p, plan.rp);
 }
 template <int EPI>
-cudaError_t gemm_go_rows(bool f8, RowsPlan const &plan, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tw,
+cudaError_t gemm_go_rows(bool f8, StreamScope const &on, RowsPlan const &plan, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tw,
 						 x17::GemmParams const &p) {
-	return f8 ? gemm_go_rows_kind<EPI, true>(plan, stream, ta, tw, p) : gemm_go_rows_kind<EPI, false>(plan, stream, ta, tw, p);
+	return f8 ? gemm_go_rows_kind<EPI, true>(on, plan, stream, ta, tw, p) : gemm_go_rows_kind<EPI, false>(on, plan, stream, ta, tw, p);
 }
 
-template <int EPI>
-cudaError_t gemm_go(bool f8, dim3 grid, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tb,
-					x17::GemmParams const &p) {
+template <int EPI, bool F8>
+cudaError_t gemm_go_kind(StreamScope const &on, dim3 grid, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tb,
+						 x17::GemmParams const &p) {
 	uint32_t const smem = x17::gemm_cfg::SMEM_BYTES;
-	cudaError_t ce;
-	if (f8) {
-		ce = cudaFuncSetAttribute(x17::gemm_kernel<EPI, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-		if (ce != cudaSuccess) return ce;
-		x17::gemm_kernel<EPI, true><<<grid, x17::gemm_cfg::THREADS, smem, stream>>>(ta, tb, p);
-	} else {
-		ce = cudaFuncSetAttribute(x17::gemm_kernel<EPI, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-		if (ce != cudaSuccess) return ce;
-		x17::gemm_kernel<EPI, false><<<grid, x17::gemm_cfg::THREADS, smem, stream>>>(ta, tb, p);
-	}
+	cudaError_t const ce = allow_smem(Kernel<&x17::gemm_kernel<EPI, F8>>{}, on.device, smem);
+	if (ce != cudaSuccess) return ce;
+	x17::gemm_kernel<EPI, F8><<<grid, x17::gemm_cfg::THREADS, smem, stream>>>(ta, tb, p);
 	return cudaSuccess;
+}
+template <int EPI>
+cudaError_t gemm_go(bool f8, StreamScope const &on, dim3 grid, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tb,
+					x17::GemmParams const &p) {
+	return f8 ? gemm_go_kind<EPI, true>(on, grid, stream, ta, tb, p) : gemm_go_kind<EPI, false>(on, grid, stream, ta, tb, p);
 }
 
 __global__ void split_i8_weights_kernel(int8_t const *w, uint64_t rows, uint64_t cols, uint8_t *out) {
@@ -1303,10 +1312,10 @@ x17ai_DiagnosticBuffer *x17ai_b200_gemm_fwd(
 	cudaError_t ce;
 	auto go = [&](auto epi) {
 		constexpr int EPI = decltype(epi)::value;
-		if (few) return gemm_go_rows<EPI>(plan.f8, few, s, ta, tb, p);
-		if (split) return gemm_go_split<EPI>(plan.f8, split, s, ta, tb, p);
-		if (pair) return gemm_go_pair<EPI>(plan.f8, scope.state().sm_count, s, ta, tb, p);
-		return gemm_go<EPI>(plan.f8, grid, s, ta, tb, p);
+		if (few) return gemm_go_rows<EPI>(plan.f8, scope, few, s, ta, tb, p);
+		if (split) return gemm_go_split<EPI>(plan.f8, scope, split, s, ta, tb, p);
+		if (pair) return gemm_go_pair<EPI>(plan.f8, scope, s, ta, tb, p);
+		return gemm_go<EPI>(plan.f8, scope, grid, s, ta, tb, p);
 	};
 	switch (plan.epi) {
 	case x17::EPI_SCALE_I8: ce = go(std::integral_constant<int, x17::EPI_SCALE_I8>{}); break;
@@ -1390,10 +1399,10 @@ x17ai_DiagnosticBuffer *x17ai_b200_qkvg_fwd_i8(
 	uint32_t const n_tiles = p.tiles_m * p.tiles_n;
 	uint32_t const ctas = n_tiles < uint32_t(scope.state().sm_count) ? n_tiles : uint32_t(scope.state().sm_count);
 	cudaError_t const ce =
-		few ? gemm_go_rows<x17::EPI_QKVG>(false, few, reinterpret_cast<cudaStream_t>(stream), ta, tb, p)
-		: split ? gemm_go_split<x17::EPI_QKVG>(false, split, reinterpret_cast<cudaStream_t>(stream), ta, tb, p)
-		: pair ? gemm_go_pair<x17::EPI_QKVG>(false, scope.state().sm_count, reinterpret_cast<cudaStream_t>(stream), ta, tb, p)
-			 : gemm_go<x17::EPI_QKVG>(false, dim3(ctas), reinterpret_cast<cudaStream_t>(stream), ta, tb, p);
+		few ? gemm_go_rows<x17::EPI_QKVG>(false, scope, few, reinterpret_cast<cudaStream_t>(stream), ta, tb, p)
+		: split ? gemm_go_split<x17::EPI_QKVG>(false, scope, split, reinterpret_cast<cudaStream_t>(stream), ta, tb, p)
+		: pair ? gemm_go_pair<x17::EPI_QKVG>(false, scope, reinterpret_cast<cudaStream_t>(stream), ta, tb, p)
+			 : gemm_go<x17::EPI_QKVG>(false, scope, dim3(ctas), reinterpret_cast<cudaStream_t>(stream), ta, tb, p);
 	if (ce != cudaSuccess) {
 		return make_diag("x17ai_b200: cudaFuncSetAttribute failed", who, ": cudaFuncSetAttribute failed: ",
 						 cudaGetErrorString(ce));

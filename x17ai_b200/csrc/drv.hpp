@@ -19,6 +19,7 @@
 	X(cuCtxPushCurrent)           \
 	X(cuCtxPopCurrent)            \
 	X(cuCtxGetDevice)             \
+	X(cuCtxGetCurrent)            \
 	X(cuStreamCreate)             \
 	X(cuStreamDestroy)            \
 	X(cuStreamSynchronize)        \

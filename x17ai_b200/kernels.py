@@ -37,6 +37,18 @@ def _ptr(t):
     return 0 if t is None else t.data_ptr()
 
 
+def _launched(native) -> bool:
+    """What a native launch (csrc/hostcall.cpp) answered: None = launched, False = some argument is irregular (the
+    Python checks below the call name it, or take what they accept), else a diagnostic. The native path takes 1 to 2 us
+    of host time off the launch's own, the Python checks and ctypes 4 to 7."""
+    if native is None:
+        return True
+    if native is False:
+        return False
+    check(native)
+    return True
+
+
 def matrix_shape(op, name, t, expected, dtype):
     """tensor_check::matrix_shape (tensor_check.rs:19-60)."""
     shape = tuple(t.shape)
@@ -117,8 +129,10 @@ class AttnKernel:
     def __init__(self, config: AttnKernelConfig):
         self.config = config
         self._lib = _lib.load()
+        self._native = _lib.hostcall()
         meta = _lib.AttnMeta()
-        cfg = config._c()
+        cfg = self._cfg = config._c()
+        self._cfg_addr = ctypes.addressof(cfg)
         check(self._lib.x17ai_b200_attn_meta(ctypes.byref(cfg), ctypes.byref(meta)))
         self.THREADS_PER_BLOCK = int(meta.threads_per_block)
         self.SMEM_BYTES = int(meta.smem_bytes)
@@ -149,6 +163,8 @@ class AttnKernel:
         return batch, seq_len
 
     def launch(self, stream, q, kv, sink_k, sink_v, attn_temperature, out, l=None, window_size=0):
+        if _launched(self._native.attn(self._cfg_addr, stream.handle, q, kv, sink_k, sink_v, attn_temperature, out, l, window_size)):
+            return
         batch, seq_len = self._shapes(q, kv, sink_k, sink_v, attn_temperature, out, l)
         cfg = self.config._c()
         check(self._lib.x17ai_b200_attn_fwd_i8(
@@ -229,6 +245,9 @@ class AttnKernel:
 
     def launch_pv_fp8(self, stream, q, kv, sink_k, sink_v, attn_temperature, v_scale, out, l=None, window_size=0):
         """fp8 P.V variant: kv holds int8 K and e4m3 V bytes (int8 view), sink_v e4m3, out bf16."""
+        if _launched(self._native.attn_pv_fp8(self._cfg_addr, stream.handle, q, kv, sink_k, sink_v, attn_temperature, v_scale, out, l,
+                                              window_size)):
+            return
         c = self.config
         batch = q.shape[0] if q.dim() == 3 else 1
         q2, kv2, out2 = (q[0], kv[0], out[0]) if q.dim() == 3 else (q, kv, out)
@@ -248,6 +267,9 @@ class AttnKernel:
                       window_size=0):
         """Inputs with one f32 scale per token and head (value = scale * code; `q_scale`, `k_scale`, `v_scale`
         f32 [B, H, S] or [H, S]), bf16 output: x17ai_b200_attn_fwd_i8_scaled."""
+        if _launched(self._native.attn_scaled(self._cfg_addr, stream.handle, q, q_scale, kv, k_scale, v_scale, sink_k, sink_v,
+                                              attn_temperature, out, l, window_size)):
+            return
         c = self.config
         batch = q.shape[0] if q.dim() == 3 else 1
         q2, kv2, out2 = (q[0], kv[0], out[0]) if q.dim() == 3 else (q, kv, out)
@@ -283,6 +305,9 @@ class AttnKernel:
         """One new token per sequence: q [B, q_stride], kv_cache [B, T, kv_stride], out [B, o_stride].
         `no_alloc=True` takes the entry point that keeps its split-KV partials in the library's built-in
         4 MiB scratch instead of allocating (see x17ai_b200_attn_decode_i8_noalloc in the header)."""
+        if _launched(self._native.decode(self._cfg_addr, stream.handle, q, kv_cache, kv_len, sink_k, sink_v, attn_temperature, out, l,
+                                         window_size, kv_lens, n_splits, no_alloc)):
+            return
         c = self.config
         batch, _ = matrix_shape("decode", "q", q, (None, c.q_stride), DTYPE_INT8)
         if kv_cache.dim() != 3 or kv_cache.shape[0] != batch or kv_cache.shape[2] != c.kv_stride:
@@ -337,8 +362,10 @@ class GemmKernel:
     def __init__(self, config: GemmConfig):
         self.config = config
         self._lib = _lib.load()
+        self._native = _lib.hostcall()
         meta = _lib.GemmMeta()
-        cfg = config._c()
+        cfg = self._cfg = config._c()
+        self._cfg_addr = ctypes.addressof(cfg)
         check(self._lib.x17ai_b200_gemm_meta(ctypes.byref(cfg), ctypes.byref(meta)))
         self.THREADS_PER_BLOCK = int(meta.threads_per_block)
         self.SMEM_BYTES = int(meta.smem_bytes)
@@ -346,6 +373,8 @@ class GemmKernel:
         self.N_PER_BLOCK = int(meta.n_per_block)
 
     def launch(self, stream, a, b, c, rrms=None, residual=None):
+        if _launched(self._native.gemm(self._cfg_addr, stream.handle, a, b, c, rrms, residual)):
+            return
         g = self.config
         a_rows = self.check_shapes(a, b, c, rrms, residual)
         cfg = g._c()
@@ -382,6 +411,8 @@ def _proj_scale(inputs: int) -> float:
 
 def qkvg_fwd_i8(stream, x, w_qkvg, n_heads, head_dim, q, kv, k_rrms, g=None, eps=2.0 ** -70):
     """Fused Q / KV / gate projection (attn_q_fwd + attn_kv_fwd of src/main.rs:387-491 in one launch)."""
+    if _launched(_lib.hostcall().qkvg(stream.handle, x, w_qkvg, n_heads, head_dim, q, kv, k_rrms, g, eps)):
+        return
     rows, model_dim = matrix_shape("qkvg", "x", x, (None, None), DTYPE_INT8)
     hd = n_heads * head_dim
     gate_cols = 0 if g is None else g.shape[1]
@@ -406,6 +437,8 @@ def split_i8_weights(stream, w):
 
 def rms_norm(stream, mode, inp, out, row_scale=None, eps=2.0 ** -70):
     """Rms_norm::kernel (rms_norm.cu:55-113) and its bf16-input modes."""
+    if _launched(_lib.hostcall().rms_norm(stream.handle, mode, inp, out, row_scale, eps)):
+        return
     in_dtype = DTYPE_E4M3 if mode == RMS_E4M3_FIXED else DTYPE_BF16
     rows, cols = matrix_shape("rms_norm", "inp", inp, (None, None), in_dtype)
     matrix_shape("rms_norm", "out", out, (rows, cols), DTYPE_INT8)
