@@ -358,6 +358,7 @@ X17_DEV void attn_fwd_body(CUtensorMap const *tm_q_ptr, CUtensorMap const *tm_kv
 		// no "empty" wait is needed, and their latency runs under the TMEM allocation
 		tma_prefetch_desc(tm_q_ptr);
 		tma_prefetch_desc(tm_kv_ptr);
+		pdl_wait();
 		mbar_expect_tx(q_full_bar, BQ * D);
 		tma_load_3d(s_q, tm_q_ptr, q_full_bar, i32(head * D), i32(q0), i32(batch));
 		for (u32 s = 0; s < n_early; ++s) {
@@ -368,12 +369,16 @@ X17_DEV void attn_fwd_body(CUtensorMap const *tm_q_ptr, CUtensorMap const *tm_kv
 	}
 	if (warp == 1) {
 		tmem_alloc(tmem_slot, TMEM_COLS);
-		if (!more_calls) tmem_relinquish();
+		if (!more_calls) {
+			tmem_relinquish();
+			pdl_launch_dependents();   // no TMEM allocation follows
+		}
 	}
 	tc_fence_before();
 	__syncthreads();
 	tc_fence_after();
 	u32 const tmem_base = *tmem_slot_gen;
+	pdl_wait();
 
 	if (warp == 0) {
 		// ---------------- TMA producer ----------------

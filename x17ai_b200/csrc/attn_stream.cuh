@@ -204,6 +204,8 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
 	__syncthreads();
 	tc_fence_after();
 	u32 const tmem_base = *tmem_slot_gen;
+	pdl_launch_dependents();
+	pdl_wait();
 
 	// item -> (batch, head, first and one-past-last query tile)
 	// the last chunks of a sequence come first: with a window the first chunk is the lightest (its

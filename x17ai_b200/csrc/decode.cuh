@@ -129,6 +129,7 @@ attn_decode_kernel(const DecodeParams p) {
 	u32 const grp = lane / LPR;        // which row of the instruction this lane works on
 	u32 const sub = lane % LPR;        // which 16-byte chunk of the row
 
+	pdl_wait();
 	u32 const kv_len = p.kv_lens ? min(p.kv_lens[batch], p.kv_capacity) : p.kv_len;
 	u32 const w = p.window;
 	u32 const k_lo = (w == 0xFFFFFFFFu || kv_len < w) ? 0u : kv_len - w;
@@ -295,6 +296,7 @@ attn_decode_kernel(const DecodeParams p) {
 			}
 		}
 	}
+	pdl_launch_dependents();   // not earlier: a next decode's clusters would be packed onto the few SMs with room
 	if (p.n_splits > 1) {
 		if (p.scratch != nullptr) return;
 		cluster_arrive();
@@ -322,6 +324,8 @@ attn_decode_merge_kernel(const DecodeParams p) {
 	u32 const head = blockIdx.x;
 	u32 const batch = blockIdx.y;
 	u32 const d = threadIdx.x;
+	pdl_launch_dependents();
+	pdl_wait();
 	u32 const kv_len = p.kv_lens ? min(p.kv_lens[batch], p.kv_capacity) : p.kv_len;
 	u32 const w = p.window;
 	u32 const n_att = (kv_len < w ? kv_len : w) + 4u;

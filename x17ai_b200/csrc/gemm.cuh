@@ -265,6 +265,8 @@ X17_DEV void gemm_body(CUtensorMap const *tm_a_ptr, CUtensorMap const *tm_b_ptr,
 	__syncthreads();
 	if constexpr (PAIR) cluster_sync_all();   // the peer's barriers are initialised before anything signals them
 	tc_fence_after();
+	pdl_launch_dependents();
+	pdl_wait();
 	u32 const tmem_base = *tmem_slot_gen;
 
 	u32 const tiles_m = PAIR ? (p.m + TILE_M - 1) / TILE_M : p.tiles_m;
@@ -516,16 +518,22 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 		tmem_alloc(tmem_slot, ACC_COLS);
 		tmem_relinquish();
 	}
+	if (threadIdx.x == 0) {
+		// the first weights start on their way to L2 while the kernel in front of this one finishes
+		tma_prefetch_desc(&tm_a);
+		tma_prefetch_desc(&tm_b);
+		for (u32 i = 0; i < 2 * sp.stages && kb_begin + i < kb_end; ++i) tma_prefetch_2d(&tm_b, i32((kb_begin + i) * BK), i32(n0));
+	}
 	tc_fence_before();
 	__syncthreads();
 	tc_fence_after();
 	u32 const tmem_base = *tmem_slot_gen;
+	pdl_launch_dependents();
+	pdl_wait();
 
 	bool ok = true;
 	if (warp == 0) {
 		if (elect_one()) {
-			tma_prefetch_desc(&tm_a);
-			tma_prefetch_desc(&tm_b);
 			for (u32 kb = kb_begin, s = 0, ph = 0; kb < kb_end; ++kb) {
 				if (!mbar_wait(empty_bar(s), ph ^ 1, ctx, ST_WAIT_STAGE_EMPTY, s)) break;
 				u32 const a_dst = smem_base + s * stage_bytes;

@@ -85,16 +85,22 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 		tmem_alloc(tmem_slot, tmem_cols);
 		tmem_relinquish();
 	}
+	if (threadIdx.x == 0) {
+		// the first weights start on their way to L2 while the kernel in front of this one finishes
+		tma_prefetch_desc(&tm_a);
+		tma_prefetch_desc(&tm_w);
+		for (u32 i = 0; i < 2 * rp.stages && kb_begin + i < kb_end; ++i) tma_prefetch_2d(&tm_w, i32((kb_begin + i) * BK), i32(w0));
+	}
 	tc_fence_before();
 	__syncthreads();
 	tc_fence_after();
 	u32 const tmem_base = *tmem_slot_gen;
+	pdl_launch_dependents();
+	pdl_wait();
 
 	bool ok = true;
 	if (warp == 0) {
 		if (elect_one()) {
-			tma_prefetch_desc(&tm_a);
-			tma_prefetch_desc(&tm_w);
 			for (u32 kb = kb_begin, s = 0, ph = 0; kb < kb_end; ++kb) {
 				if (!mbar_wait(empty_bar(s), ph ^ 1, ctx, ST_WAIT_STAGE_EMPTY, s)) break;
 				u32 const dst = smem_base + s * st_bytes;

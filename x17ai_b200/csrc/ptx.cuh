@@ -71,6 +71,18 @@ X17_DEV bool elect_one() {
 	return pred != 0;
 }
 
+// Programmatic dependent launch. Every kernel of the library calls pdl_launch_dependents() once its CTA holds what it
+// allocates (TMEM: a dependent CTA on the same SM that took the columns first and then waited for this grid would wait
+// for ever), and pdl_wait() before its first access to global memory: the next kernel's set-up (launch, barriers, TMEM,
+// descriptor fetches) then runs under the tail of this one, and no kernel touches data before the grids in front of it
+// have completed. Without the launch attribute both are no-ops.
+X17_DEV void pdl_launch_dependents() {
+	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+X17_DEV void pdl_wait() {
+	asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 X17_DEV f32 ex2_approx(f32 x) {
 	f32 r;
 	asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -251,6 +263,10 @@ X17_DEV void tma_load_3d(u32 dst, CUtensorMap const *map, u32 bar, i32 x, i32 y,
 		:
 		: "r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z)
 		: "memory");
+}
+// brings a tile into L2 (reads no data into the SM: safe before pdl_wait, whoever writes the tile)
+X17_DEV void tma_prefetch_2d(CUtensorMap const *map, i32 x, i32 y) {
+	asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
 }
 X17_DEV void tma_prefetch_desc(CUtensorMap const *map) {
 	asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");

@@ -259,12 +259,16 @@ X17_DEV void rms_norm_body_keep(RmsParams const &p) {
 
 __global__ void __launch_bounds__(rms_cfg::THREADS)
 rms_norm_keep_kernel(const RmsParams p) {
+	pdl_launch_dependents();
+	pdl_wait();
 	rms_norm_body_keep(p);
 }
 
 template <int MODE>
 __global__ void __launch_bounds__(rms_cfg::THREADS)
 rms_norm_kernel(const RmsParams p) {
+	pdl_launch_dependents();
+	pdl_wait();
 	rms_norm_body<MODE>(p);
 }
 
