@@ -158,125 +158,105 @@ X17_DEV void extreme_chunk(u32 const (&r)[32], u32 col0, u32 lo, u32 span, i32 (
 // quantised probabilities: P = rint(255 * 2^(x - m) * v_scale[key] / g), g = the largest v_scale among the row's
 // visible keys, so that P <= 255, P.V stays an exact u8 x s8 product and out = O * g / (255 * sum).
 // The first sweep reduces t = acc * k_scale[key] (the row maximum of x is a_row times its largest, or for a negative
-// temperature its smallest, value) and v_scale; the second computes the probabilities of 32 columns.
-template <bool EDGE, bool WANT_MAX>
-X17_DEV void scaled_extreme_chunk(u32 const (&r)[32], u32 col0, u32 key0, u32 seq_len, f32 const *ksc, f32 const *vsc,
-								  u32 lo, u32 span, f32 &t_ext, f32 &v_max) {
-#pragma unroll
-	for (u32 i = 0; i < 32; ++i) {
-		u32 const key = key0 + i;
-		bool vis = key < seq_len;
-		if constexpr (EDGE) vis = vis && (col0 + i - lo) < span;
-		if (vis) {
-			f32 const t = __fmul_rn(__int2float_rn(i32(r[i])), __ldg(ksc + key));
-			t_ext = WANT_MAX ? fmaxf(t_ext, t) : fminf(t_ext, t);
-			v_max = fmaxf(v_max, __ldg(vsc + key));
-		}
-	}
-}
-template <bool EDGE>
-X17_DEV void scaled_softmax_chunk(u32 const (&r)[32], u32 col0, u32 key0, u32 seq_len, f32 a_row, f32 const *ksc,
-								  f32 const *vsc, f32 neg_m, f32 rg, u32 lo, u32 span, f32 &sum, u32 (&pk)[8]) {
-	using namespace attn_cfg;
-#pragma unroll
-	for (u32 g = 0; g < 8; ++g) {
-		u32 q4[4];
-#pragma unroll
-		for (u32 e4 = 0; e4 < 4; ++e4) {
-			u32 const i = 4 * g + e4;
-			u32 const key = key0 + i;
-			bool vis = key < seq_len;
-			if constexpr (EDGE) vis = vis && (col0 + i - lo) < span;
-			f32 pq = 0.0f;
-			if (vis) {
-				f32 const t = __fmul_rn(__int2float_rn(i32(r[i])), __ldg(ksc + key));
-				f32 const e = ex2_approx(__fmaf_rn(t, a_row, neg_m));
-				sum = __fadd_rn(sum, e);
-				pq = fminf(__fmul_rn(__fmul_rn(e, __ldg(vsc + key)), rg), 255.0f);
-			}
-			q4[e4] = __float_as_uint(__fadd_rn(pq, MAGIC));   // rint(pq) in the low byte
-		}
-		u32 const lo2 = __byte_perm(q4[0], q4[1], 0x0040);
-		u32 const hi2 = __byte_perm(q4[2], q4[3], 0x0040);
-		pk[g] = __byte_perm(lo2, hi2, 0x5410);
-	}
-}
+// temperature its smallest, value) and v_scale; the second computes the probabilities.
+//
+// A scale belongs to a column of the score tile. With one thread per row every lane of a warp needs every column's
+// scale: a 16-byte load of one address by 32 lanes puts 512 bytes into registers, four cycles of the SM's load path,
+// and the 64 of them per warp and tile that the two sweeps need kept that path busy for 2048 cycles per CTA and tile
+// (the exponentials take 1024). So this mode reads the scores in the 16x256b shape: a lane holds the column pairs
+// 8 j + 2 (lane % 4) + {0, 1} of the rows lane / 4 + 8 i, i = 0 .. 3 ("slots"): 16 columns of four rows instead of 64
+// of one, a quarter of the loads, and eight bytes per load do, which every even alignment allows. Row sums and maxima
+// are finished by two shuffles per slot and sweep; P leaves as 2-byte stores (free of bank conflicts: the eight rows of
+// a store lie in different 16-byte chunks of the swizzle).
+// Measured: 8 x 32 heads x 8192 x 128, window 1024 2.54 -> 2.06 ms; 2 x 32 x 7001 x 128 (whose odd rows had taken a path of
+// single loads with a test per key) 810 -> 472 us; 2 x 64 x 8192 x 64, no window 3.85 -> 2.88 ms. What is left above the
+// FixedI8 kernel (1.14 ms) is issue slots: 2 instructions per score against 0.4 in the first sweep, 5.8 against 4.2 in the second.
+constexpr u32 FRAG_ROWS = 4;   // rows of a thread's score fragment
+X17_DEV u32 frag_row(u32 slot, u32 lane) { return 8 * slot + lane / 4; }   // inside the warp's 32 rows
 
-// The same two helpers for a tile that every row sees whole and whose scale vectors can be read four keys at a
-// time (16-byte aligned: seq_len a multiple of 4): no masks, no bounds checks (the tile lies below the diagonal,
-// so its keys exist), a quarter of the loads, and the multiplications and additions as packed f32x2 instructions;
-// the values are those of the general helpers (the same operations in the same order per element).
-// EDGE: the tile lies inside the sequence but the row sees only columns lo <= col < lo + span of it
-template <bool WANT_MAX, bool EDGE = false>
-X17_DEV void scaled_extreme_chunk_full(u32 const (&r)[32], f32 const *ksc, f32 const *vsc, f32 &t_ext, f32 &v_max,
-									   u32 col0 = 0, u32 lo = 0, u32 span = 0) {
+// N column pairs' scales: keys key + 8 j + {0, 1}. IN_PAIRS: `sc + key` is 8-byte aligned and every key exists.
+template <u32 N>
+X17_DEV void load_scale_pairs(f32 const *sc, u32 key, u32 seq_len, bool in_pairs, u64 (&out)[N]) {
+	if (in_pairs) {
 #pragma unroll
-	for (u32 g = 0; g < 8; ++g) {
-		float4 const k4 = __ldg(reinterpret_cast<float4 const *>(ksc) + g);
-		float4 v4 = __ldg(reinterpret_cast<float4 const *>(vsc) + g);
-		f32 t0, t1, t2, t3;
-		unpack_f32x2(mul_f32x2(pack_f32x2(__int2float_rn(i32(r[4 * g])), __int2float_rn(i32(r[4 * g + 1]))),
-							   pack_f32x2(k4.x, k4.y)), t0, t1);
-		unpack_f32x2(mul_f32x2(pack_f32x2(__int2float_rn(i32(r[4 * g + 2])), __int2float_rn(i32(r[4 * g + 3]))),
-							   pack_f32x2(k4.z, k4.w)), t2, t3);
-		if constexpr (EDGE) {
-			f32 const none = WANT_MAX ? -INFINITY : INFINITY;
-			bool const s0 = (col0 + 4 * g - lo) < span, s1 = (col0 + 4 * g + 1 - lo) < span;
-			bool const s2 = (col0 + 4 * g + 2 - lo) < span, s3 = (col0 + 4 * g + 3 - lo) < span;
-			t0 = s0 ? t0 : none; t1 = s1 ? t1 : none; t2 = s2 ? t2 : none; t3 = s3 ? t3 : none;
-			v4.x = s0 ? v4.x : 0.0f; v4.y = s1 ? v4.y : 0.0f; v4.z = s2 ? v4.z : 0.0f; v4.w = s3 ? v4.w : 0.0f;
+		for (u32 j = 0; j < N; ++j) {
+			float2 const v = __ldg(reinterpret_cast<float2 const *>(sc + key + 8 * j));
+			out[j] = pack_f32x2(v.x, v.y);
 		}
-		if constexpr (WANT_MAX) {
-			t_ext = fmaxf(fmaxf(t_ext, t0), t1);
-			t_ext = fmaxf(fmaxf(t_ext, t2), t3);
-		} else {
-			t_ext = fminf(fminf(t_ext, t0), t1);
-			t_ext = fminf(fminf(t_ext, t2), t3);
+	} else {
+		u32 const last = seq_len - 1;
+#pragma unroll
+		for (u32 j = 0; j < N; ++j) {
+			out[j] = pack_f32x2(__ldg(sc + min(key + 8 * j, last)), __ldg(sc + min(key + 8 * j + 1, last)));
 		}
-		v_max = fmaxf(fmaxf(v_max, v4.x), v4.y);
-		v_max = fmaxf(fmaxf(v_max, v4.z), v4.w);
 	}
 }
-template <bool EDGE = false>
-X17_DEV void scaled_softmax_chunk_full(u32 const (&r)[32], f32 a_row, f32 const *ksc, f32 const *vsc, f32 neg_m, f32 rg,
-									   f32 &sum, u32 (&pk)[8], u32 col0 = 0, u32 lo = 0, u32 span = 0) {
+// The 32 rows x 32 columns at `taddr` in fragment form: r[slot / 2][4 j + 2 (slot % 2) + {0, 1}].
+X17_DEV void load_frag(u32 taddr, u32 (&r)[2][16]) {
+	tmem_ld_16x256b_x4(taddr, r[0]);
+	tmem_ld_16x256b_x4(taddr + (16u << 16), r[1]);
+}
+X17_DEV u64 frag_pair(u32 const (&r)[16], u32 slot, u32 j) {
+	u32 const i = 4 * j + 2 * (slot & 1);
+	return pack_f32x2(__int2float_rn(i32(r[i])), __int2float_rn(i32(r[i + 1])));
+}
+// EDGE: a row sees the keys at distance `dist` = row - 1 - key with u32(dist) < wlim; `dist[slot]` is that of the
+// fragment's first column. `sgn` is -1 where the smallest value is wanted.
+template <bool EDGE>
+X17_DEV void scaled_extreme_frag(u32 const (&r)[2][16], u64 const *ks, u64 const *vs, u64 sgn, i32 const (&dist)[FRAG_ROWS], u32 wlim,
+								 f32 (&t_ext)[FRAG_ROWS], f32 (&v_max)[FRAG_ROWS]) {
+#pragma unroll
+	for (u32 j = 0; j < 4; ++j) {
+		u64 const k2 = mul_f32x2(ks[j], sgn);
+		f32 v0 = 0.0f, v1 = 0.0f;
+		if constexpr (EDGE) unpack_f32x2(vs[j], v0, v1);
+#pragma unroll
+		for (u32 s = 0; s < FRAG_ROWS; ++s) {
+			f32 t0, t1;
+			unpack_f32x2(mul_f32x2(frag_pair(r[s >> 1], s, j), k2), t0, t1);
+			if constexpr (EDGE) {
+				bool const s0 = u32(dist[s] - i32(8 * j)) < wlim, s1 = u32(dist[s] - i32(8 * j + 1)) < wlim;
+				t0 = s0 ? t0 : -INFINITY;
+				t1 = s1 ? t1 : -INFINITY;
+				v_max[s] = fmaxf(fmaxf(v_max[s], s0 ? v0 : 0.0f), s1 ? v1 : 0.0f);
+			}
+			t_ext[s] = fmaxf(fmaxf(t_ext[s], t0), t1);
+		}
+	}
+}
+// Slots s0 and s0 + 1. pk[slot - s0][j]: the two bytes of column pair j
+template <bool EDGE>
+X17_DEV void scaled_softmax_frag(u32 s0, u32 const (&r)[16], u64 const *ks, u64 const *vs, f32 const (&a_row)[FRAG_ROWS],
+								 f32 const (&neg_m)[FRAG_ROWS], f32 const (&rg)[FRAG_ROWS], i32 const (&dist)[FRAG_ROWS], u32 wlim,
+								 u64 (&sum2)[FRAG_ROWS], u32 (&pk)[2][4]) {
 	using namespace attn_cfg;
-	u64 const arow2 = pack_f32x2(a_row, a_row);
-	u64 const negm2 = pack_f32x2(neg_m, neg_m);
-	u64 const rg2 = pack_f32x2(rg, rg);
 	u64 const magic2 = pack_f32x2(MAGIC, MAGIC);
-	u64 sum2 = pack_f32x2(sum, 0.0f);
 #pragma unroll
-	for (u32 g = 0; g < 8; ++g) {
-		float4 const k4 = __ldg(reinterpret_cast<float4 const *>(ksc) + g);
-		float4 const v4 = __ldg(reinterpret_cast<float4 const *>(vsc) + g);
-		u32 q4[4];
+	for (u32 s = s0; s < s0 + 2; ++s) {
+		u64 const a2 = pack_f32x2(a_row[s], a_row[s]), m2 = pack_f32x2(neg_m[s], neg_m[s]), g2 = pack_f32x2(rg[s], rg[s]);
 #pragma unroll
-		for (u32 h = 0; h < 2; ++h) {
-			u64 const kk = h == 0 ? pack_f32x2(k4.x, k4.y) : pack_f32x2(k4.z, k4.w);
-			u64 const vv = h == 0 ? pack_f32x2(v4.x, v4.y) : pack_f32x2(v4.z, v4.w);
-			u64 const t2 = mul_f32x2(pack_f32x2(__int2float_rn(i32(r[4 * g + 2 * h])), __int2float_rn(i32(r[4 * g + 2 * h + 1]))), kk);
+		for (u32 j = 0; j < 4; ++j) {
 			f32 x0, x1;
-			unpack_f32x2(fma_f32x2(t2, arow2, negm2), x0, x1);
+			unpack_f32x2(fma_f32x2(mul_f32x2(frag_pair(r, s, j), ks[j]), a2, m2), x0, x1);
+			bool see0 = true, see1 = true;
 			if constexpr (EDGE) {   // ex2(-inf) = 0: no weight, no share of the sum
-				x0 = (col0 + 4 * g + 2 * h - lo) < span ? x0 : -INFINITY;
-				x1 = (col0 + 4 * g + 2 * h + 1 - lo) < span ? x1 : -INFINITY;
+				see0 = u32(dist[s] - i32(8 * j)) < wlim;
+				see1 = u32(dist[s] - i32(8 * j + 1)) < wlim;
+				x0 = see0 ? x0 : -INFINITY;
+				x1 = see1 ? x1 : -INFINITY;
 			}
 			u64 const e2 = pack_f32x2(ex2_approx(x0), ex2_approx(x1));
-			sum2 = add_f32x2(sum2, e2);
-			// e * v_scale * (255 / g) <= 255 up to rounding, so no clamp: rint lands in the low mantissa byte
+			sum2[s] = add_f32x2(sum2[s], e2);
+			// x <= 0 (m is rounded up), so e * v_scale * (255 / g) <= 255 up to rounding: rint lands in the low byte
 			f32 qa, qb;
-			unpack_f32x2(fma_f32x2(mul_f32x2(e2, vv), rg2, magic2), qa, qb);
-			q4[2 * h] = __float_as_uint(qa);
-			q4[2 * h + 1] = __float_as_uint(qb);
+			unpack_f32x2(fma_f32x2(mul_f32x2(e2, vs[j]), g2, magic2), qa, qb);
+			if constexpr (EDGE) {   // (an unseen key's scale may be anything)
+				qa = see0 ? qa : MAGIC;
+				qb = see1 ? qb : MAGIC;
+			}
+			pk[s - s0][j] = __byte_perm(__float_as_uint(qa), __float_as_uint(qb), 0x0040);
 		}
-		u32 const lo2 = __byte_perm(q4[0], q4[1], 0x0040);
-		u32 const hi2 = __byte_perm(q4[2], q4[3], 0x0040);
-		pk[g] = __byte_perm(lo2, hi2, 0x5410);
 	}
-	f32 s0, s1;
-	unpack_f32x2(sum2, s0, s1);
-	sum = __fadd_rn(s0, s1);
 }
 
 // FP8PV: P.V on the fp8 tensor path (P as e4m3 of 256 * p, V as e4m3 with a per-head f32 scale, f32
@@ -518,10 +498,9 @@ X17_DEV void attn_fwd_body(CUtensorMap const *tm_q_ptr, CUtensorMap const *tm_kv
 		f32 const a_row = SCALED ? __fmul_rn(__fmul_rn(temp, 64.0f), row_ok ? __ldg(p.tok_q_scale + tok_base + qi) : 0.125f) : 0.0f;
 		f32 const *const ksc = SCALED ? p.tok_k_scale + tok_base : nullptr;
 		f32 const *const vsc = SCALED ? p.tok_v_scale + tok_base : nullptr;
-		// whole tiles may read the scale vectors four keys at a time when every (batch, head) row of them starts
-		// on a 16-byte boundary
-		bool const scales_by_four = SCALED && (p.seq_len & 3u) == 0
-									&& ((reinterpret_cast<u64>(p.tok_k_scale) | reinterpret_cast<u64>(p.tok_v_scale)) & 15u) == 0;
+		// tiles whose keys all exist read the scale vectors two keys at a time when this (batch, head)'s start on an
+		// 8-byte boundary
+		bool const scales_by_two = SCALED && ((reinterpret_cast<u64>(ksc) | reinterpret_cast<u64>(vsc)) & 7u) == 0;
 		// the head's sink values as f32 and its sink key, once per CTA (the key is read after sweep 1, one
 		// named barrier later; the values in the epilogue)
 		if (threadIdx.x - 64u < D) {
@@ -546,10 +525,31 @@ X17_DEV void attn_fwd_body(CUtensorMap const *tm_q_ptr, CUtensorMap const *tm_kv
 		i32 ext[4];
 #pragma unroll
 		for (u32 i = 0; i < 4; ++i) ext[i] = pos_t ? INT32_MIN : INT32_MAX;
-		f32 t_ext = pos_t ? -INFINITY : INFINITY, v_max = 0.0f;  // per-token-scale mode: extreme of acc * k_scale, largest v_scale
+		// per-token-scale mode: the fragment's column 0 and rows (see load_frag above), per slot the extreme of acc * k_scale
+		// (the largest value of its negative where the temperature is negative) and the largest v_scale of edge tiles
+		u32 const frag_col = col_base + 2 * (lane & 3u);
+		u32 const wlim = min(w, 0x7FFFFFFFu);
+		f32 t_ext[FRAG_ROWS] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, v_max[FRAG_ROWS] = {0.0f, 0.0f, 0.0f, 0.0f};
+		f32 v_all = 0.0f;   // of the tiles that every row sees: this lane's two columns
+		auto frag_dist = [&](u32 k0, i32 (&dist)[FRAG_ROWS]) {
+#pragma unroll
+			for (u32 s = 0; s < FRAG_ROWS; ++s) dist[s] = i32(q0 + quarter * 32 + frag_row(s, lane)) - 1 - i32(k0 + frag_col);
+		};
 		#pragma unroll 1
 		for (u32 t = t_begin; t <= t_end && ok; ++t) {
+			u32 const k0 = t * BKV;
+			bool const edge = (t == t_end) || (w != 0xFFFFFFFFu && k0 + w < q0 + BQ - 1);
 			u32 const b = (t - t_begin) & 1u;
+			// the scales are requested ahead of the wait for the scores
+			u64 ks[SCALED ? 8 : 1];
+			f32 va = 0.0f, vb = 0.0f;
+			if constexpr (SCALED) {
+				load_scale_pairs(ksc, k0 + frag_col, p.seq_len, scales_by_two && k0 + BKV <= p.seq_len, ks);
+				if (!edge) {
+					va = __ldg(vsc + k0 + col_base + lane);
+					vb = __ldg(vsc + k0 + col_base + 32 + lane);
+				}
+			}
 			u32 const par = b == 0 ? (use0 & 1u) : (use1 & 1u);
 			if (!mbar_wait_warp(s_full_bar(b), par, ctx, ST_WAIT_S_FULL, t)) {
 				ok = false;
@@ -558,8 +558,30 @@ X17_DEV void attn_fwd_body(CUtensorMap const *tm_q_ptr, CUtensorMap const *tm_kv
 			use0 += b == 0 ? 1u : 0u;
 			use1 += b == 0 ? 0u : 1u;
 			tc_fence_after();
-			u32 const k0 = t * BKV;
-			bool const edge = (t == t_end) || (w != 0xFFFFFFFFu && k0 + w < q0 + BQ - 1);
+			if constexpr (SCALED) {
+				u64 const sgn = pos_t ? pack_f32x2(1.0f, 1.0f) : pack_f32x2(-1.0f, -1.0f);
+				if (!edge) v_all = fmaxf(fmaxf(v_all, va), vb);
+#pragma unroll
+				for (u32 ch = 0; ch < 2; ++ch) {
+					u32 f[2][16];
+					load_frag(tmem_base + lane_addr + b * BKV + col_base + 32 * ch, f);
+					tmem_wait_ld();
+					if (ch == 1) {
+						tc_fence_before();
+						mbar_arrive(s_done_bar(b));  // S_b is in registers now
+					}
+					i32 dist[FRAG_ROWS];
+					if (!edge) {
+						scaled_extreme_frag<false>(f, ks + 4 * ch, ks, sgn, dist, wlim, t_ext, v_max);
+					} else {
+						u64 vs[4];
+						load_scale_pairs(vsc, k0 + frag_col + 32 * ch, p.seq_len, scales_by_two && k0 + BKV <= p.seq_len, vs);
+						frag_dist(k0 + 32 * ch, dist);
+						scaled_extreme_frag<true>(f, ks + 4 * ch, vs, sgn, dist, wlim, t_ext, v_max);
+					}
+				}
+				continue;
+			}
 			u32 lo = 0, span = BKV;
 			if (edge) visible(k0, lo, span);
 			u32 r0[32], r1[32];
@@ -569,40 +591,7 @@ X17_DEV void attn_fwd_body(CUtensorMap const *tm_q_ptr, CUtensorMap const *tm_kv
 			tmem_wait_ld();
 			tc_fence_before();
 			mbar_arrive(s_done_bar(b));  // S_b is in registers now
-			if constexpr (SCALED) {
-				u32 const kc = k0 + col_base;
-				if (edge && scales_by_four && k0 + BKV <= p.seq_len) {   // an edge tile whose keys all exist
-					if (pos_t) {
-						scaled_extreme_chunk_full<true, true>(r0, ksc + kc, vsc + kc, t_ext, v_max, col_base, lo, span);
-						scaled_extreme_chunk_full<true, true>(r1, ksc + kc + 32, vsc + kc + 32, t_ext, v_max, col_base + 32, lo, span);
-					} else {
-						scaled_extreme_chunk_full<false, true>(r0, ksc + kc, vsc + kc, t_ext, v_max, col_base, lo, span);
-						scaled_extreme_chunk_full<false, true>(r1, ksc + kc + 32, vsc + kc + 32, t_ext, v_max, col_base + 32, lo, span);
-					}
-				} else if (edge) {
-					if (pos_t) {
-						scaled_extreme_chunk<true, true>(r0, col_base, kc, p.seq_len, ksc, vsc, lo, span, t_ext, v_max);
-						scaled_extreme_chunk<true, true>(r1, col_base + 32, kc + 32, p.seq_len, ksc, vsc, lo, span, t_ext, v_max);
-					} else {
-						scaled_extreme_chunk<true, false>(r0, col_base, kc, p.seq_len, ksc, vsc, lo, span, t_ext, v_max);
-						scaled_extreme_chunk<true, false>(r1, col_base + 32, kc + 32, p.seq_len, ksc, vsc, lo, span, t_ext, v_max);
-					}
-				} else if (scales_by_four) {
-					if (pos_t) {
-						scaled_extreme_chunk_full<true>(r0, ksc + kc, vsc + kc, t_ext, v_max);
-						scaled_extreme_chunk_full<true>(r1, ksc + kc + 32, vsc + kc + 32, t_ext, v_max);
-					} else {
-						scaled_extreme_chunk_full<false>(r0, ksc + kc, vsc + kc, t_ext, v_max);
-						scaled_extreme_chunk_full<false>(r1, ksc + kc + 32, vsc + kc + 32, t_ext, v_max);
-					}
-				} else if (pos_t) {
-					scaled_extreme_chunk<false, true>(r0, col_base, kc, p.seq_len, ksc, vsc, lo, span, t_ext, v_max);
-					scaled_extreme_chunk<false, true>(r1, col_base + 32, kc + 32, p.seq_len, ksc, vsc, lo, span, t_ext, v_max);
-				} else {
-					scaled_extreme_chunk<false, false>(r0, col_base, kc, p.seq_len, ksc, vsc, lo, span, t_ext, v_max);
-					scaled_extreme_chunk<false, false>(r1, col_base + 32, kc + 32, p.seq_len, ksc, vsc, lo, span, t_ext, v_max);
-				}
-			} else if (!edge) {
+			if (!edge) {
 				if (pos_t) {
 					extreme_chunk<false, true>(r0, col_base, lo, span, ext);
 					extreme_chunk<false, true>(r1, col_base + 32, lo, span, ext);
@@ -638,8 +627,30 @@ X17_DEV void attn_fwd_body(CUtensorMap const *tm_q_ptr, CUtensorMap const *tm_kv
 								: min(min(ext[0], ext[1]), min(ext[2], ext[3]));
 			if (e != (pos_t ? INT32_MIN : INT32_MAX)) cand = __fmul_rn(__int2float_rn(e), temp);
 		}
-		if constexpr (SCALED) cand = (t_ext > -INFINITY && t_ext < INFINITY) ? __fmul_rn(t_ext, a_row) : -INFINITY;
-		xchg[xid] = cand;
+		// per-token-scale mode: [half][row] extremes and value scales, then [row] (a_row, -m, 255 / g), in the P buffer,
+		// which nothing uses before the second sweep
+		f32 *const frag_x = reinterpret_cast<f32 *>(smem_gen + BQ * D + STAGES * TILE_BYTES);
+		if constexpr (SCALED) {
+			// the four lanes of a row, and for v_all the whole warp
+#pragma unroll
+			for (u32 o = 16; o > 0; o >>= 1) v_all = fmaxf(v_all, __shfl_xor_sync(0xffffffffu, v_all, o));
+			f32 my_t = 0.0f, my_v = 0.0f;
+#pragma unroll
+			for (u32 s = 0; s < FRAG_ROWS; ++s) {
+#pragma unroll
+				for (u32 o = 1; o < 4; o <<= 1) {
+					t_ext[s] = fmaxf(t_ext[s], __shfl_xor_sync(0xffffffffu, t_ext[s], o));
+					v_max[s] = fmaxf(v_max[s], __shfl_xor_sync(0xffffffffu, v_max[s], o));
+				}
+				my_t = (lane & 3u) == s ? t_ext[s] : my_t;
+				my_v = (lane & 3u) == s ? v_max[s] : my_v;
+			}
+			u32 const my_row = quarter * 32 + frag_row(lane & 3u, lane);
+			frag_x[half * BQ + my_row] = my_t;
+			frag_x[2 * BQ + half * BQ + my_row] = fmaxf(my_v, v_all);
+		} else {
+			xchg[xid] = cand;
+		}
 		named_barrier_sync(1, ROW_THREADS);   // also: sks has been written
 		// sink score: exact int32 dot product of this row's q with sink_k (the sink key and value are FixedI8,
 		// scale 1/8, in every mode). q comes from the Q tile in shared memory, after the first sweep: reading the
@@ -663,34 +674,99 @@ X17_DEV void attn_fwd_body(CUtensorMap const *tm_q_ptr, CUtensorMap const *tm_kv
 		}
 		f32 const sink_s = SCALED ? __fmul_rn(__fmul_rn(__int2float_rn(sink_dot), a_row), 0.125f)
 								  : __fmul_rn(__int2float_rn(sink_dot), temp);
-		f32 const m = fmaxf(sink_s, fmaxf(cand, xchg[xpartner]));
-		named_barrier_sync(1, ROW_THREADS);  // the exchange area is reused for the sums
-		// per-token-scale mode: g = the row's largest v_scale; P = 255 * 2^(x - m) * v_scale / g
-		f32 g_row = 0.0f, rg = 0.0f;
+		// per-token-scale mode: g = the largest v_scale among the row's visible keys; P = 255 * 2^(x - m) * v_scale / g
+		f32 g_row = 0.0f;
+		f32 fa[FRAG_ROWS], fm[FRAG_ROWS], fg[FRAG_ROWS];   // a_row, -m and 255 / g of the fragment's rows
 		if constexpr (SCALED) {
-			xchg[xid] = v_max;
-			named_barrier_sync(1, ROW_THREADS);
-			g_row = fmaxf(v_max, xchg[xpartner]);   // the largest v_scale among the row's visible keys
-			named_barrier_sync(1, ROW_THREADS);
-			if (g_row > 0.0f) rg = __fmul_rn(255.0f, rcp_approx(g_row));
+			f32 const te = fmaxf(frag_x[row], frag_x[BQ + row]);
+			g_row = fmaxf(frag_x[2 * BQ + row], frag_x[3 * BQ + row]);
+			// rounded up: no x = fma(t, a_row, -m) is above zero, so no P above 255
+			cand = (te > -INFINITY && te < INFINITY) ? __fmul_ru(pos_t ? te : -te, a_row) : -INFINITY;
+		} else {
+			cand = fmaxf(cand, xchg[xpartner]);
 		}
+		f32 const m = fmaxf(sink_s, cand);
+		if constexpr (SCALED) {
+			if (half == 0) {
+				frag_x[4 * BQ + row] = a_row;
+				frag_x[5 * BQ + row] = -m;
+				frag_x[6 * BQ + row] = g_row > 0.0f ? __fmul_rn(255.0f, rcp_approx(g_row)) : 0.0f;
+			}
+			named_barrier_sync(1, ROW_THREADS);
+#pragma unroll
+			for (u32 s = 0; s < FRAG_ROWS; ++s) {
+				f32 const *const fx = frag_x + 4 * BQ + quarter * 32 + frag_row(s, lane);
+				fa[s] = fx[0];
+				fm[s] = fx[BQ];
+				fg[s] = fx[2 * BQ];
+			}
+		}
+		named_barrier_sync(1, ROW_THREADS);  // the exchange area is reused for the sums, the P buffer for P
 
 		// ---- sweep 2: probabilities against the final maximum ----
 		f32 const neg_m = -m;
 		f32 sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+		u64 fsum[FRAG_ROWS] = {0, 0, 0, 0};   // per-token-scale mode: two f32 sums per slot
 		u32 const p_row = s_p + row * 128u;
 		u32 const sw = row & 7u;
 		u32 const ch0 = half * 4u;  // first of this thread's four 16-byte chunks
 		#pragma unroll 1
 		for (u32 t = t_begin; t <= t_end && ok; ++t) {
+			u32 const k0 = t * BKV;
+			bool const edge = (t == t_end) || (w != 0xFFFFFFFFu && k0 + w < q0 + BQ - 1);
+			if constexpr (SCALED) {
+				bool const in_pairs = scales_by_two && k0 + BKV <= p.seq_len;
+				u64 ks[4], vs[4];
+				load_scale_pairs(ksc, k0 + frag_col, p.seq_len, in_pairs, ks);   // ahead of the wait for the scores
+				load_scale_pairs(vsc, k0 + frag_col, p.seq_len, in_pairs, vs);
+				ok = mbar_wait_warp(s_full_bar(0), use0 & 1, ctx, ST_WAIT_S_FULL, t);
+				++use0;
+				tc_fence_after();
+#pragma unroll
+				for (u32 ch = 0; ch < 2 && ok; ++ch) {
+					u32 f[2][16];
+					load_frag(tmem_base + lane_addr + col_base + 32 * ch, f);
+					tmem_wait_ld();
+					if (ch == 1) {
+						tc_fence_before();
+						mbar_arrive(s_done_bar(0));  // S has been read: the next Q.K^T may overwrite it
+					}
+					i32 dist[FRAG_ROWS];
+					frag_dist(k0 + 32 * ch, dist);
+#pragma unroll
+					for (u32 s0 = 0; s0 < FRAG_ROWS; s0 += 2) {
+						u32 pk[2][4];
+						if (edge) scaled_softmax_frag<true>(s0, f[s0 >> 1], ks, vs, fa, fm, fg, dist, wlim, fsum, pk);
+						else scaled_softmax_frag<false>(s0, f[s0 >> 1], ks, vs, fa, fm, fg, dist, wlim, fsum, pk);
+						if (ch == 0 && s0 == 0 && t > t_begin) {   // P.V of the previous tile has finished reading the P buffer
+							ok = mbar_wait_warp(pv_done_bar, (t - t_begin - 1) & 1, ctx, ST_WAIT_O_FULL, 0x100u + t);
+							if (!ok) break;
+						}
+#pragma unroll
+						for (u32 s = s0; s < s0 + 2; ++s) {
+							u32 const fr = quarter * 32 + frag_row(s, lane);
+#pragma unroll
+							for (u32 j = 0; j < 4; ++j) {
+								st_shared_u16(s_p + fr * 128u + (((half * 4u + ch * 2u + j / 2) ^ (fr & 7u)) << 4) + 8 * (j & 1u) + 2 * (lane & 3u), pk[s - s0][j]);
+							}
+						}
+					}
+					if (ch == 0) {
+						load_scale_pairs(ksc, k0 + frag_col + 32, p.seq_len, in_pairs, ks);
+						load_scale_pairs(vsc, k0 + frag_col + 32, p.seq_len, in_pairs, vs);
+					}
+				}
+				if (!ok) break;
+				fence_proxy_async_smem();
+				mbar_arrive(p_ready_bar);
+				continue;
+			}
 			if (!mbar_wait_warp(s_full_bar(0), use0 & 1, ctx, ST_WAIT_S_FULL, t)) {
 				ok = false;
 				break;
 			}
 			++use0;
 			tc_fence_after();
-			u32 const k0 = t * BKV;
-			bool const edge = (t == t_end) || (w != 0xFFFFFFFFu && k0 + w < q0 + BQ - 1);
 			u32 lo = 0, span = BKV;
 			if (edge) visible(k0, lo, span);
 			u32 r0[32], r1[32];
@@ -701,21 +777,7 @@ X17_DEV void attn_fwd_body(CUtensorMap const *tm_q_ptr, CUtensorMap const *tm_kv
 			tmem_wait_ld();
 			tc_fence_before();
 			mbar_arrive(s_done_bar(0));  // S is in registers: the next Q.K^T may overwrite it
-			if constexpr (SCALED) {
-				if (edge && scales_by_four && k0 + BKV <= p.seq_len) {
-					scaled_softmax_chunk_full<true>(r0, a_row, ksc + k0 + col_base, vsc + k0 + col_base, neg_m, rg, sum[0], pk0, col_base, lo, span);
-					scaled_softmax_chunk_full<true>(r1, a_row, ksc + k0 + col_base + 32, vsc + k0 + col_base + 32, neg_m, rg, sum[1], pk1, col_base + 32, lo, span);
-				} else if (edge) {
-					scaled_softmax_chunk<true>(r0, col_base, k0 + col_base, p.seq_len, a_row, ksc, vsc, neg_m, rg, lo, span, sum[0], pk0);
-					scaled_softmax_chunk<true>(r1, col_base + 32, k0 + col_base + 32, p.seq_len, a_row, ksc, vsc, neg_m, rg, lo, span, sum[1], pk1);
-				} else if (scales_by_four) {
-					scaled_softmax_chunk_full(r0, a_row, ksc + k0 + col_base, vsc + k0 + col_base, neg_m, rg, sum[0], pk0);
-					scaled_softmax_chunk_full(r1, a_row, ksc + k0 + col_base + 32, vsc + k0 + col_base + 32, neg_m, rg, sum[1], pk1);
-				} else {
-					scaled_softmax_chunk<false>(r0, col_base, k0 + col_base, p.seq_len, a_row, ksc, vsc, neg_m, rg, lo, span, sum[0], pk0);
-					scaled_softmax_chunk<false>(r1, col_base + 32, k0 + col_base + 32, p.seq_len, a_row, ksc, vsc, neg_m, rg, lo, span, sum[1], pk1);
-				}
-			} else if (!edge) {
+			if (!edge) {
 				softmax_chunk<false, FP8PV>(r0, col_base, temp, neg_m, lo, span, sum, pk0);
 				softmax_chunk<false, FP8PV>(r1, col_base + 32, temp, neg_m, lo, span, sum, pk1);
 			} else {
@@ -748,9 +810,24 @@ X17_DEV void attn_fwd_body(CUtensorMap const *tm_q_ptr, CUtensorMap const *tm_kv
 		}
 
 		// ---- normalise and store: each thread of the pair takes half of the D columns ----
-		f32 const part = __fadd_rn(__fadd_rn(sum[0], sum[1]), __fadd_rn(sum[2], sum[3]));
-		xchg[xid] = part;
+		f32 part = __fadd_rn(__fadd_rn(sum[0], sum[1]), __fadd_rn(sum[2], sum[3]));
+		if constexpr (SCALED) {
+			f32 mine = 0.0f;
+#pragma unroll
+			for (u32 s = 0; s < FRAG_ROWS; ++s) {
+				f32 a, b;
+				unpack_f32x2(fsum[s], a, b);
+				a = __fadd_rn(a, b);
+				a = __fadd_rn(a, __shfl_xor_sync(0xffffffffu, a, 1));
+				a = __fadd_rn(a, __shfl_xor_sync(0xffffffffu, a, 2));
+				mine = (lane & 3u) == s ? a : mine;
+			}
+			xchg[half * BQ + quarter * 32 + frag_row(lane & 3u, lane)] = mine;
+		} else {
+			xchg[xid] = part;
+		}
 		named_barrier_sync(1, ROW_THREADS);
+		if constexpr (SCALED) part = xchg[xid];
 		f32 const other = xchg[xpartner];
 		f32 const both = half == 0 ? __fadd_rn(part, other) : __fadd_rn(other, part);
 		if (ok && mbar_wait_warp(o_full_bar, 0, ctx, ST_WAIT_O_FULL, 0)) {

@@ -240,6 +240,10 @@ X17_DEV void st_shared_v4(u32 addr, u32 a, u32 b, u32 c, u32 d) {
 				 : "memory");
 }
 
+X17_DEV void st_shared_u16(u32 addr, u32 v) {
+	asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"(static_cast<unsigned short>(v)) : "memory");
+}
+
 // generic-proxy writes to shared memory -> visible to the async proxy (TMA, tcgen05.mma)
 X17_DEV void fence_proxy_async_smem() {
 	asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -397,6 +401,17 @@ X17_DEV void tmem_ld_32x32b_x32(u32 taddr, u32 (&r)[32]) {
 }
 
 // 32 lanes x 16 columns
+// 16 lanes x 32 columns: r[4 j + 2 h + b] is lane `thread` / 4 + 8 h, column 8 j + 2 (`thread` % 4) + b
+X17_DEV void tmem_ld_16x256b_x4(u32 taddr, u32 (&r)[16]) {
+	asm volatile(
+		"tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+		"{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+		: "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+		  "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+		  "=r"(r[14]), "=r"(r[15])
+		: "r"(taddr)
+		: "memory");
+}
 X17_DEV void tmem_ld_32x32b_x16(u32 taddr, u32 (&r)[16]) {
 	asm volatile(
 		"tcgen05.ld.sync.aligned.32x32b.x16.b32 "
