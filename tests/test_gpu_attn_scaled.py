@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from oracle import attn as o_attn
-from test_gpu_attn import _launch_scaled, _scaled_case
+from test_gpu_attn import _launch, _launch_scaled, _scaled_case
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +38,30 @@ def test_scales_of_unseen_keys_do_not_matter(stream):
     seen = np.zeros(S, dtype=bool)
     seen[41:41 + W] = True
     assert np.array_equal(got[:, ~seen], want[:, ~seen])
+
+
+def test_large_scores_give_the_fixedi8_probabilities(stream):
+    """With every scale 1/8 and a score maximum of 2^12 to 2^15 (long q and k that differ in a few entries: the ulp of the
+    maximum is a visible part of a probability step) P is that of the FixedI8 kernel. Values are one-hot per key, with one
+    more dimension that sums P: the ratio of two bf16 outputs is P / sum(P) to twice the bf16 rounding of 2^-8."""
+    rng = np.random.default_rng(5)
+    B, H, D, S = 1, 8, 128, 64
+    q = np.full((B, S, H, D), 127, dtype=np.int8)
+    k = np.full((B, S, H, D), 127, dtype=np.int8)
+    q[..., :8] = rng.integers(1, 5, (B, S, H, 8))
+    k[..., :8] -= rng.integers(0, 30, (B, S, H, 8)).astype(np.int8)
+    v = np.zeros((B, S, H, D), dtype=np.int8)
+    v[:, np.arange(S), :, np.arange(S)] = 127
+    v[..., 127] = 127
+    sk = np.zeros((H, D), dtype=np.int8)
+    temp = np.linspace(0.5, 1.9, H).astype(np.float32)
+    kv = np.concatenate((k, v), axis=-1).reshape(B, S, 2 * H * D)
+    _, l, _, p, _ = _launch(stream, q.reshape(B, S, H * D), kv, sk, sk, temp, H, D, 0, debug=True)
+    assert 2.0 ** 12 < l[:, :, 32:].min() and l.max() < 2.0 ** 15
+    eighth = np.full((B, H, S), 0.125, dtype=np.float32)
+    got, _ = _launch_scaled(stream, (q, eighth), (k, eighth), (v, eighth), sk, sk, temp, H, D, 0)
+    for h in range(H):
+        for i in range(1, S):
+            want = p[h, i, :i] / p[h, i, :i].sum(dtype=np.float64)
+            ratio = got[0, i, h, :i] / got[0, i, h, 127].astype(np.float64)
+            assert np.all(np.abs(ratio - want) <= (2.0 ** -7 + 2.0 ** -14) * want), (h, i)

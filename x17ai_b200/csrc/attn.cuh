@@ -186,6 +186,14 @@ X17_DEV void extreme_chunk(u32 const (&r)[32], u32 col0, u32 lo, u32 span, i32 (
 // single loads with a test per key) 810 -> 472 us; 2 x 64 x 8192 x 64, no window 3.85 -> 2.88 ms. What is left above the
 // FixedI8 kernel (1.14 ms) is issue slots: 2 instructions per score against 0.4 in the first sweep, 5.8 against 4.2 in the second.
 constexpr u32 FRAG_ROWS = 4;   // rows of a thread's score fragment
+
+// The row maximum m, to nearest as every mode has it (rounded up, all of a row's x move by up to an ulp of m, and 1 to 2 %
+// more error against 64 bits comes out where the scores are large). The largest x = fma(t, a, -m) may then be half an ulp
+// of m above zero: below |m| = 2^16 that leaves rint(255 * 2^x) at 255, from there on m is rounded up instead.
+X17_DEV f32 largest_score(f32 t, f32 a) {
+	f32 const m = __fmul_rn(t, a);
+	return fabsf(m) < 65536.0f ? m : __fmul_ru(t, a);
+}
 X17_DEV u32 frag_row(u32 slot, u32 lane) { return 8 * slot + lane / 4; }   // inside the warp's 32 rows
 
 // N column pairs' scales: keys key + 8 j + {0, 1}. IN_PAIRS: `sc + key` is 8-byte aligned and every key exists.
@@ -261,7 +269,7 @@ X17_DEV void scaled_softmax_frag(u32 s0, u32 const (&r)[16], u64 const *ks, u64 
 			}
 			u64 const e2 = pack_f32x2(ex2_approx(x0), ex2_approx(x1));
 			sum2[s] = add_f32x2(sum2[s], e2);
-			// x <= 0 (m is rounded up), so e * v_scale * (255 / g) <= 255 up to rounding: rint lands in the low byte
+			// e * v_scale * (255 / g) < 255.5 (see largest_score): rint lands in the low byte
 			f32 qa, qb;
 			unpack_f32x2(fma_f32x2(mul_f32x2(e2, vs[j]), g2, magic2), qa, qb);
 			if constexpr (EDGE) {   // (an unseen key's scale may be anything)
@@ -694,8 +702,7 @@ X17_DEV void attn_fwd_body(CUtensorMap const *tm_q_ptr, CUtensorMap const *tm_kv
 		if constexpr (SCALED) {
 			f32 const te = fmaxf(frag_x[row], frag_x[BQ + row]);
 			g_row = fmaxf(frag_x[2 * BQ + row], frag_x[3 * BQ + row]);
-			// rounded up: no x = fma(t, a_row, -m) is above zero, so no P above 255
-			cand = (te > -INFINITY && te < INFINITY) ? __fmul_ru(pos_t ? te : -te, a_row) : -INFINITY;
+			cand = (te > -INFINITY && te < INFINITY) ? largest_score(pos_t ? te : -te, a_row) : -INFINITY;
 		} else {
 			cand = fmaxf(cand, xchg[xpartner]);
 		}
