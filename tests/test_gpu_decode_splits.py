@@ -32,3 +32,28 @@ def test_decode_split_forms(stream, D, kv_len, W, splits):
         # P is rounded against running maxima here, against the final one in the oracle: at most one code apart
         assert hist[2:].sum() == 0 and hist[1] / ref_out.size <= 0.08, hist
         assert np.max(np.abs(l.cpu().numpy() - ref_l)) <= 1e-3
+
+
+@pytest.mark.parametrize("D,splits", [(32, 2), (64, 8), (128, 3), (128, 8), (128, 40)])
+def test_decode_splits_without_keys(stream, D, splits):
+    """A ragged batch of lengths 0 to 33: most splits have no key at all and their CTAs reach the merge before the first
+    CTA of the cluster has read its keys. Launched repeatedly, behind one another: every launch gives the same bytes."""
+    from x17ai_b200 import kernels as K
+    B, H, T = 12, 5, 64
+    rng = np.random.default_rng(D + splits)
+    q, kv, sk, sv, temp = _case(rng, B, H, D, T)
+    lens = np.array([0, 1, 2, 15, 16, 17, 0, 31, 32, 33, 1, 5], dtype=np.int32)
+    kern = K.AttnKernel(K.AttnKernelConfig(H, D, H * D, 2 * H * D, H * D))
+    dev = [torch.from_numpy(a).cuda() for a in (q, kv, sk, sv, temp, lens)]
+    outs = torch.zeros((50, B, H * D), dtype=torch.int8, device="cuda")
+    ls = torch.zeros((50, B, H), dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    for i in range(50):
+        kern.decode(stream, dev[0], dev[1], T, dev[2], dev[3], dev[4], outs[i], ls[i], kv_lens=dev[5], n_splits=splits)
+    stream.synchronize()
+    assert (outs == outs[0]).all() and (ls == ls[0]).all()
+    for b in range(B):
+        ref_out, ref_l = o_attn.attn_decode_i8(q[b:b + 1], kv[b:b + 1], int(lens[b]), sk, sv, temp, 0, H, D, kv_tile=1 << 20)
+        hist = code_hist(outs[0, b:b + 1].cpu().numpy(), ref_out)
+        assert hist[2:].sum() == 0, (b, hist)   # P is rounded against running maxima here: at most one code apart
+        assert np.max(np.abs(ls[0, b].cpu().numpy() - ref_l[0])) <= 1e-3

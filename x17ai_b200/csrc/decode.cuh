@@ -129,6 +129,7 @@ attn_decode_kernel(const DecodeParams p) {
 	u32 const grp = lane / LPR;        // which row of the instruction this lane works on
 	u32 const sub = lane % LPR;        // which 16-byte chunk of the row
 
+	cluster_arrive();   // "this CTA runs" (a launch without clusters is one of single CTAs)
 	pdl_wait();
 	u32 const kv_len = p.kv_lens ? min(p.kv_lens[batch], p.kv_capacity) : p.kv_len;
 	u32 const w = p.window;
@@ -155,6 +156,10 @@ attn_decode_kernel(const DecodeParams p) {
 	extern __shared__ f32 partials[];   // first CTA of a cluster: [n_splits][D + 2]
 
 	f32 fm = 0.0f, fs = 0.0f, fo = 0.0f;   // of the CTA's split, in the threads below D
+	// Shared memory of another CTA may be written only once that CTA is known to run; being scheduled together is not enough,
+	// and a split without keys gets to its store within a few hundred cycles. (Asked for at entry: 5.51 -> 5.54 us a call for
+	// one sequence of 1500 keys. Behind a branch on the launch's form the loop spilled a register: 2 %.)
+	cluster_wait();
 	#pragma unroll 1
 	for (u32 split = blockIdx.z; split < p.n_splits; split += gridDim.z) {
 		u32 const s_lo = k_lo + split * per_split;
@@ -299,7 +304,8 @@ attn_decode_kernel(const DecodeParams p) {
 	pdl_launch_dependents();   // not earlier: a next decode's clusters would be packed onto the few SMs with room
 	if (p.n_splits > 1) {
 		if (p.scratch != nullptr) return;
-		cluster_arrive();
+		__syncwarp();
+		cluster_arrive();              // this CTA's partials are stored
 		if (blockIdx.z != 0) return;   // its slot is free for the next CTA: only the first CTA waits
 		cluster_wait();
 	}
