@@ -252,6 +252,13 @@ X17_DEV void gemm_body(CUtensorMap const *tm_a_ptr, CUtensorMap const *tm_b_ptr,
 		*abort_flag = 0;
 		mbar_fence_init();
 	}
+	// tcgen05.alloc.cta_group::2 works on both CTAs' TMEM: the peer has to be running. Launched under the tail of another
+	// kernel the two may start a microsecond apart (32 ns or less in half of the launches, then up to 1.2 us), and where one
+	// had allocated 0.9 us before the other began, the other's allocation never returned.
+	if constexpr (PAIR) {
+		__syncwarp();
+		cluster_sync_all();
+	}
 	if (warp == 1) {
 		if constexpr (PAIR) {
 			tmem_alloc_pair(tmem_slot, 512);
@@ -263,7 +270,7 @@ X17_DEV void gemm_body(CUtensorMap const *tm_a_ptr, CUtensorMap const *tm_b_ptr,
 	}
 	tc_fence_before();
 	__syncthreads();
-	if constexpr (PAIR) cluster_sync_all();   // the peer's barriers are initialised before anything signals them
+	if constexpr (PAIR) cluster_sync_all();   // both have allocated: the first CTA's MMAs write the peer's TMEM too
 	tc_fence_after();
 	pdl_launch_dependents();
 	pdl_wait();
@@ -441,6 +448,10 @@ X17_DEV void gemm_body(CUtensorMap const *tm_a_ptr, CUtensorMap const *tm_b_ptr,
 		tc_fence_after();
 		if constexpr (PAIR) tmem_dealloc_pair(tmem_base, 512);
 		else tmem_dealloc(tmem_base, 512);
+	}
+	if constexpr (PAIR) {   // the same for the release: neither CTA makes room for another kernel's before both have released
+		__syncwarp();
+		cluster_sync_all();
 	}
 }
 
