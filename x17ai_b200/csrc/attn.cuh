@@ -202,14 +202,13 @@ X17_DEV void load_scale_pairs(f32 const *sc, u32 key, u32 seq_len, bool in_pairs
 	if (in_pairs) {
 #pragma unroll
 		for (u32 j = 0; j < N; ++j) {
-			float2 const v = __ldg(reinterpret_cast<float2 const *>(sc + key + 8 * j));
-			out[j] = pack_f32x2(v.x, v.y);
+			out[j] = ld_global_f32x2(sc + key + 8 * j);
 		}
 	} else {
 		u32 const last = seq_len - 1;
 #pragma unroll
 		for (u32 j = 0; j < N; ++j) {
-			out[j] = pack_f32x2(__ldg(sc + min(key + 8 * j, last)), __ldg(sc + min(key + 8 * j + 1, last)));
+			out[j] = pack_f32x2(ld_global(sc + min(key + 8 * j, last)), ld_global(sc + min(key + 8 * j + 1, last)));
 		}
 	}
 }
@@ -512,14 +511,14 @@ X17_DEV void attn_fwd_body(CUtensorMap const *tm_q_ptr, CUtensorMap const *tm_kv
 		u32 const n_att = (qi < w ? qi : w) + 4u;
 		f32 const base_t = f32((1.0 / 64.0) * (D == 128 ? 0.08838834764831845 : D == 64 ? 0.125 : 0.17677669529663687));
 		f32 const row_t = __fmul_rn(base_t, lg2_approx(f32(n_att)));
-		f32 const head_t = __ldg(p.temperature + head);
+		f32 const head_t = p.temperature[head];
 		f32 const temp = __fmul_rn(row_t, head_t);
 		bool const pos_t = head_t >= 0.0f;  // uniform over the CTA; row_t > 0 always
 		// per-token-scale mode: x = acc * a_row * k_scale[key]; the FixedI8 mode is its case q_scale = k_scale = 1/8
 		u64 const tok_base = (u64(batch) * p.n_heads + head) * p.seq_len;
-		f32 const a_row = SCALED ? __fmul_rn(__fmul_rn(temp, 64.0f), row_ok ? __ldg(p.tok_q_scale + tok_base + qi) : 0.125f) : 0.0f;
-		f32 const *const ksc = SCALED ? p.tok_k_scale + tok_base : nullptr;
-		f32 const *const vsc = SCALED ? p.tok_v_scale + tok_base : nullptr;
+		f32 const a_row = SCALED ? __fmul_rn(__fmul_rn(temp, 64.0f), row_ok ? p.tok_q_scale[tok_base + qi] : 0.125f) : 0.0f;
+		f32 const *const ksc = SCALED ? behind_wait(p.tok_k_scale) + tok_base : nullptr;
+		f32 const *const vsc = SCALED ? behind_wait(p.tok_v_scale) + tok_base : nullptr;
 		// tiles whose keys all exist read the scale vectors two keys at a time when this (batch, head)'s start on an
 		// 8-byte boundary
 		bool const scales_by_two = SCALED && ((reinterpret_cast<u64>(ksc) | reinterpret_cast<u64>(vsc)) & 7u) == 0;
@@ -568,8 +567,8 @@ X17_DEV void attn_fwd_body(CUtensorMap const *tm_q_ptr, CUtensorMap const *tm_kv
 			if constexpr (SCALED) {
 				load_scale_pairs(ksc, k0 + frag_col, p.seq_len, scales_by_two && k0 + BKV <= p.seq_len, ks);
 				if (!edge) {
-					va = __ldg(vsc + k0 + col_base + lane);
-					vb = __ldg(vsc + k0 + col_base + 32 + lane);
+					va = ld_global(vsc + k0 + col_base + lane);
+					vb = ld_global(vsc + k0 + col_base + 32 + lane);
 				}
 			}
 			u32 const par = b == 0 ? (use0 & 1u) : (use1 & 1u);
@@ -861,7 +860,7 @@ X17_DEV void attn_fwd_body(CUtensorMap const *tm_q_ptr, CUtensorMap const *tm_kv
 			constexpr u32 HALF_D = D / 2;
 			u32 const d0 = half * HALF_D;
 			u64 const out_off = u64(batch) * p.o_batch_stride + u64(qi) * p.o_stride + head * D + d0;
-			f32 const vs = FP8PV ? __fmul_rn(recip, __ldg(p.v_scale + head)) : recip;
+			f32 const vs = FP8PV ? __fmul_rn(recip, p.v_scale[head]) : recip;
 			// all of this thread's O columns are requested at once: one load latency per row instead of four
 			u32 r_all[HALF_D / 16][16];
 #pragma unroll

@@ -435,7 +435,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
 			for (u32 item = blockIdx.x; item < plan.n_items; item += gridDim.x) {
 				u32 batch, head, j0, j1;
 				decode_item(item, batch, head, j0, j1);
-				f32 const head_t = __ldg(p.temperature + head);
+				f32 const head_t = p.temperature[head];
 				bool const pos_t = head_t >= 0.0f;  // uniform over the item; the row factor is positive
 				// the sink values of this head as f32, one copy per row quarter (its four warps write it here and
 				// read it in the epilogues, which start one pass and one exchange barrier of the quarter later; the
@@ -607,7 +607,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
 						f32 const recip = rcp_approx(total);
 						u32 const d0 = cq * DQ;
 						u64 const out_off = u64(batch) * p.o_batch_stride + u64(qi2) * p.o_stride + head * D + d0;
-						f32 const vs = FP8PV ? __fmul_rn(recip, __ldg(p.v_scale + head)) : recip;
+						f32 const vs = FP8PV ? __fmul_rn(recip, p.v_scale[head]) : recip;
 	#pragma unroll
 						for (u32 c = 0; c < DQ; c += CH) {
 							u32 r[CH];

@@ -141,12 +141,12 @@ attn_decode_kernel(const DecodeParams p) {
 	uint4 const qv = *reinterpret_cast<uint4 const *>(p.q + u64(batch) * p.q_stride + head * D + sub * 16);
 	u32 const qw[4] = {qv.x, qv.y, qv.z, qv.w};
 	// the sink token's operands are read ahead of the stream of keys
-	uint4 const sk = __ldg(reinterpret_cast<uint4 const *>(p.sink_k + head * D + sub * 16));
+	uint4 const sk = *reinterpret_cast<uint4 const *>(p.sink_k + head * D + sub * 16);
 	f32 const sink_v = threadIdx.x < D ? f32(p.sink_v[head * D + threadIdx.x]) : 0.0f;
 
 	u32 const n_att = (kv_len < w ? kv_len : w) + 4u;
 	f32 const base_t = f32((1.0 / 64.0) * (D == 128 ? 0.08838834764831845 : D == 64 ? 0.125 : 0.17677669529663687));
-	f32 const temp = __fmul_rn(__fmul_rn(base_t, lg2_approx(f32(n_att))), __ldg(p.temperature + head));
+	f32 const temp = __fmul_rn(__fmul_rn(base_t, lg2_approx(f32(n_att))), p.temperature[head]);
 
 	i8 const *kv_base = p.kv + u64(batch) * p.kv_batch_stride + u64(head) * 2 * D + sub * 16;
 	u32 const step = WARPS * RPI * UNROLL;
@@ -177,8 +177,8 @@ attn_decode_kernel(const DecodeParams p) {
 			for (u32 u = 0; u < UNROLL; ++u) {
 				u32 const t = t0 + u * RPI + grp;
 				i8 const *rowp = kv_base + u64(t < s_hi ? t : s_lo) * p.kv_stride;
-				kq[u] = __ldg(reinterpret_cast<uint4 const *>(rowp));
-				vq[u] = __ldg(reinterpret_cast<uint4 const *>(rowp + D));
+				kq[u] = *reinterpret_cast<uint4 const *>(rowp);
+				vq[u] = *reinterpret_cast<uint4 const *>(rowp + D);
 			}
 		};
 		u32 since_flush = 0;  // an int32 accumulator takes at most 4 * 255 * 127 per step: flush long before 2^31
@@ -336,7 +336,7 @@ attn_decode_merge_kernel(const DecodeParams p) {
 	u32 const w = p.window;
 	u32 const n_att = (kv_len < w ? kv_len : w) + 4u;
 	f32 const base_t = f32((1.0 / 64.0) * (D == 128 ? 0.08838834764831845 : D == 64 ? 0.125 : 0.17677669529663687));
-	f32 const temp = __fmul_rn(__fmul_rn(base_t, lg2_approx(f32(n_att))), __ldg(p.temperature + head));
+	f32 const temp = __fmul_rn(__fmul_rn(base_t, lg2_approx(f32(n_att))), p.temperature[head]);
 
 	f32 fm, fs, fo;
 	merge_partials<D>(p.scratch + (u64(batch) * p.n_heads + head) * p.n_splits * (D + 2), p.n_splits, d, fm, fs, fo);
@@ -344,7 +344,7 @@ attn_decode_merge_kernel(const DecodeParams p) {
 	uint4 const *qh = reinterpret_cast<uint4 const *>(p.q + u64(batch) * p.q_stride + head * D);
 	uint4 const *sk = reinterpret_cast<uint4 const *>(p.sink_k + head * D);
 	for (u32 i = 0; i < D / 16; ++i) {
-		uint4 a = qh[i], b = __ldg(sk + i);
+		uint4 a = qh[i], b = sk[i];
 		sdot = __dp4a(i32(a.x), i32(b.x), sdot);
 		sdot = __dp4a(i32(a.y), i32(b.y), sdot);
 		sdot = __dp4a(i32(a.z), i32(b.z), sdot);

@@ -75,12 +75,33 @@ X17_DEV bool elect_one() {
 // allocates (TMEM: a dependent CTA on the same SM that took the columns first and then waited for this grid would wait
 // for ever), and pdl_wait() before its first access to global memory: the next kernel's set-up (launch, barriers, TMEM,
 // descriptor fetches) then runs under the tail of this one, and no kernel touches data before the grids in front of it
-// have completed. Without the launch attribute both are no-ops.
+// have completed. Without the launch attribute both are no-ops. A kernel's lifetime therefore begins before its inputs
+// are written: they are read with plain loads or TMA, never with read-only (non-coherent) loads, which want data that
+// nobody writes while the kernel lives and which the compiler may move above the wait.
 X17_DEV void pdl_launch_dependents() {
 	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 X17_DEV void pdl_wait() {
 	asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Plain loads of data that no kernel writes from pdl_wait() to this kernel's end, free to be scheduled over the memory clobbers
+// of the other instructions (ordinary C++ loads are not: 4 % of the scaled attention). `p` comes from behind_wait(), so
+// that none of them moves above the wait.
+template <typename T>
+X17_DEV T const *behind_wait(T const *p) {
+	asm volatile("" : "+l"(p)::"memory");
+	return p;
+}
+X17_DEV f32 ld_global(f32 const *p) {
+	f32 v;
+	asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+	return v;
+}
+X17_DEV u64 ld_global_f32x2(f32 const *p) {
+	u64 v;
+	asm("ld.global.b64 %0, [%1];" : "=l"(v) : "l"(p));
+	return v;
 }
 
 X17_DEV f32 ex2_approx(f32 x) {

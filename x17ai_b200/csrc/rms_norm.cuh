@@ -91,7 +91,7 @@ X17_DEV void rms_norm_body(RmsParams const &p) {
 	for (u32 s = 0; s < MAX_CHUNKS; ++s) {
 		if (s < per_lane) {
 			u32 const ci = s * 32 + lane;
-			regs[s] = ci < n_chunks ? __ldg(src + ci) : make_uint4(0, 0, 0, 0);
+			regs[s] = ci < n_chunks ? src[ci] : make_uint4(0, 0, 0, 0);
 		}
 	}
 	f32 local = 0.0f;
@@ -209,7 +209,7 @@ X17_DEV void rms_norm_body_keep(RmsParams const &p) {
 	for (u32 s = 0; s < KEEP_CHUNKS; ++s) {
 		if (s < per_lane) {
 			u32 const ci = s * 32 + lane;
-			raw[s] = ci < n_chunks ? __ldg(src + ci) : make_uint4(0, 0, 0, 0);
+			raw[s] = ci < n_chunks ? src[ci] : make_uint4(0, 0, 0, 0);
 		}
 	}
 	u32 h[KEEP_CHUNKS][8];  // the row as f16x2
