@@ -119,7 +119,10 @@ PyObject *launch(F &&call) {
 		regular = false;
 	}
 	Py_END_ALLOW_THREADS
-	if (!regular) Py_RETURN_FALSE;
+	if (!regular) {
+		PyErr_Clear();
+		Py_RETURN_FALSE;
+	}
 	if (d != nullptr) return PyLong_FromVoidPtr(d);
 	Py_RETURN_NONE;
 }
@@ -308,7 +311,19 @@ PyObject *init(PyObject *, PyObject *addresses) {
 	Py_RETURN_NONE;
 }
 
-#define X17_FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
+// Reading an argument can throw (a layout without strides, a subclass that answers from Python): no C++ exception leaves a C
+// callback, the answer is False and the Python checks raise what there is to raise.
+template <PyObject *(*F)(PyObject *, PyObject *const *, Py_ssize_t)>
+PyObject *guarded(PyObject *self, PyObject *const *a, Py_ssize_t n) noexcept {
+	try {
+		return F(self, a, n);
+	} catch (...) {
+	}
+	PyErr_Clear();
+	Py_RETURN_FALSE;
+}
+
+#define X17_FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded<name>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
 	{"init", init, METH_O, nullptr},
 	{"entries", [](PyObject *, PyObject *) -> PyObject * {
