@@ -54,3 +54,64 @@ def test_shim_error_paths(stream, lib):
     with pytest.raises(X17Error, match="cuModuleGetFunction"):
         _lib.unwrap(lib.x17ai_cuda_get_kernel(kern.module, b"no_such_kernel", 0))
     kern.unload()
+
+
+_TWO_CONTEXTS = """
+import ctypes
+import numpy as np
+from x17ai_b200 import _lib, device
+
+lib, cu = _lib.load(), ctypes.CDLL("libcuda.so.1")
+H, S, D, M = 4, 256, 128, 300
+rng = np.random.default_rng(0)
+codes = lambda *s: rng.integers(-20, 20, s, dtype=np.int8)
+q, kv, sk, temp, w = codes(S, H * D), codes(S, 2 * H * D), codes(H, D), np.ones(H, np.float32), codes(512, H * D)
+attn = _lib.AttnConfig(H, D, H * D, 2 * H * D, H * D)
+gemm = _lib.GemmConfig(0x31, 0x31, 0x51, 0, H * D, 512, 1.0, 1.0, 0.0, 0)
+
+def launches(h):
+    bufs = []
+    def up(a):
+        bufs.append(_lib.unwrap(lib.x17ai_cuda_alloc(h, a.nbytes)))
+        _lib.check(lib.x17ai_cuda_upload_data(h, a.ctypes.data, bufs[-1], 0, a.nbytes))
+        return bufs[-1]
+    outs = [np.zeros((S, H * D), np.int8), np.zeros((S, 512), np.int32), np.zeros((1, H * D), np.int8)]
+    d = [up(a) for a in (q, kv, sk, temp, w)] + [up(o) for o in outs]
+    _lib.check(lib.x17ai_b200_attn_fwd_i8(h, ctypes.byref(attn), 1, S, d[0], d[1], d[2], d[2], d[3], d[5], None, 0))
+    _lib.check(lib.x17ai_b200_gemm_fwd(h, ctypes.byref(gemm), d[0], S, d[4], 512, d[6], None, None))
+    _lib.check(lib.x17ai_b200_attn_decode_i8_noalloc(h, ctypes.byref(attn), 1, d[0], d[1], S, S, None, d[2], d[2], d[3], d[7], None, 0, 65))
+    for o, p in zip(outs, d[5:]):
+        _lib.check(lib.x17ai_cuda_download_data(h, p, o.ctypes.data, 0, o.nbytes))
+    _lib.check(lib.x17ai_cuda_synchronize(h))
+    status = (ctypes.c_uint32 * 4)()
+    _lib.check(lib.x17ai_b200_read_status(h, status))
+    assert list(status) == [0, 0, 0, 0]
+    for b in bufs:
+        _lib.check(lib.x17ai_cuda_free(h, b))
+    return outs
+
+first = device.CudaStream(0)
+want = launches(first.handle)
+assert want[1].any() and np.array_equal(want[1], q.astype(np.int32) @ w.astype(np.int32).T)
+ctx, st = ctypes.c_void_p(), ctypes.c_void_p()
+assert cu.cuCtxCreate_v2(ctypes.byref(ctx), 0, 0) == 0
+assert cu.cuStreamCreate(ctypes.byref(st), 1) == 0
+assert cu.cuCtxPopCurrent_v2(ctypes.byref(ctypes.c_void_p())) == 0
+for handle in (st.value, first.handle, st.value):
+    assert all(np.array_equal(a, b) for a, b in zip(launches(handle), want))
+first.close()
+again = device.CudaStream(0)
+assert all(np.array_equal(a, b) for a, b in zip(launches(again.handle), want))
+print("same")
+"""
+
+
+def test_two_contexts_on_one_device():
+    """A second context on the device, launches in turn from both, and the primary context opened a second time: shared
+    memory limits, status words and the built-in decode scratch belong to a context. In a process without torch's CUDA."""
+    import subprocess
+    import sys
+    from pathlib import Path
+    r = subprocess.run([sys.executable, "-c", _TWO_CONTEXTS], cwd=Path(__file__).resolve().parent.parent, capture_output=True, text=True,
+                       timeout=120)
+    assert r.returncode == 0 and r.stdout.strip() == "same", (r.returncode, r.stdout, r.stderr[-800:])

@@ -35,22 +35,56 @@ std::atomic<unsigned> g_attn_item_tiles{0};   // 0 = chosen per launch
 std::mutex g_capture_mutex;
 std::unordered_map<void *, CUcontext> g_capture_ctx;   // streams between graph_begin and graph_end
 
-// ---- per-device state -----------------------------------------------------------------------
+// ---- per-context state -----------------------------------------------------------------------
 
 constexpr int MAX_DEVICES = 32;
-struct DeviceState {
-	std::once_flag once;
-	uint32_t *status = nullptr;  // 4 words of device memory
-	int sm_count = 0;
-	cudaError_t init_err = cudaSuccess;
+// Memory and function attributes belong to a context, and a device can have several: what is kept is kept per context. The
+// id is never used twice in a process (the address of a context may be). One entry per context ever launched in.
+struct ContextState {
+	uint64_t id;
+	uint32_t *status;  // 4 words of device memory
+	int sm_count;
+	ContextState *next;
 };
-DeviceState g_dev[MAX_DEVICES];
+std::atomic<ContextState *> g_contexts{nullptr};   // newest first; entries stay
+std::mutex g_contexts_mutex;                       // for adding one
+
+ContextState *find_context(uint64_t id) {
+	for (ContextState *c = g_contexts.load(std::memory_order_acquire); c != nullptr; c = c->next) {
+		if (c->id == id) return c;
+	}
+	return nullptr;
+}
+// The current context's entry; null and an error where it cannot be set up (the next call tries again).
+ContextState *context_state(uint64_t id, int device, cudaError_t &err) {
+	err = cudaSuccess;
+	if (ContextState *c = find_context(id)) return c;
+	std::lock_guard<std::mutex> lock(g_contexts_mutex);
+	if (ContextState *c = find_context(id)) return c;
+	int major = 0, sms = 0;
+	uint32_t *status = nullptr;
+	err = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device);
+	if (err == cudaSuccess && major != 10) err = cudaErrorNoKernelImageForDevice;
+	if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+	if (err == cudaSuccess) err = cudaMalloc(&status, 4 * sizeof(uint32_t));
+	if (err == cudaSuccess) err = cudaMemset(status, 0, 4 * sizeof(uint32_t));
+	auto *c = err == cudaSuccess ? new (std::nothrow) ContextState{id, status, sms, g_contexts.load(std::memory_order_relaxed)} : nullptr;
+	if (c == nullptr) {
+		if (status != nullptr) (void)cudaFree(status);
+		if (err == cudaSuccess) err = cudaErrorMemoryAllocation;
+		(void)cudaGetLastError();
+		return nullptr;
+	}
+	g_contexts.store(c, std::memory_order_release);
+	return c;
+}
 
 // Makes the stream's context current for the scope (the callers of this library keep no
 // context current, cpp/ffi.hpp:195-206) and resolves the device ordinal.
 struct StreamScope {
 	CUcontext ctx = nullptr;
 	int device = -1;
+	ContextState *context = nullptr;
 	bool pushed = false;
 	x17ai_DiagnosticBuffer *diag = nullptr;
 
@@ -84,23 +118,12 @@ struct StreamScope {
 			return;
 		}
 		device = int(dev);
-		DeviceState &st = g_dev[device];
-		std::call_once(st.once, [&] {
-			int major = 0, minor = 0;
-			cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device);
-			cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device);
-			if (major != 10) {
-				st.init_err = cudaErrorNoKernelImageForDevice;
-				return;
-			}
-			cudaDeviceGetAttribute(&st.sm_count, cudaDevAttrMultiProcessorCount, device);
-			st.init_err = cudaMalloc(&st.status, 4 * sizeof(uint32_t));
-			if (st.init_err == cudaSuccess) st.init_err = cudaMemset(st.status, 0, 4 * sizeof(uint32_t));
-		});
-		if (st.init_err != cudaSuccess) {
+		unsigned long long id = 0;
+		cudaError_t ce = cudaErrorInvalidValue;
+		if (DRV(cuCtxGetId)(ctx, &id) == CUDA_SUCCESS) context = context_state(id, device, ce);
+		if (context == nullptr) {
 			diag = make_diag("x17ai_b200: device initialisation failed", who,
-							 ": device initialisation failed (this library needs an sm_100 GPU): ",
-							 cudaGetErrorString(st.init_err));
+							 ": device initialisation failed (this library needs an sm_100 GPU): ", cudaGetErrorString(ce));
 		}
 	}
 	~StreamScope() {
@@ -109,20 +132,20 @@ struct StreamScope {
 			DRV(cuCtxPopCurrent)(&popped);
 		}
 	}
-	DeviceState &state() const { return g_dev[device]; }
+	ContextState const &state() const { return *context; }
 };
 
-// Raises a kernel's dynamic shared memory limit, once per kernel and device.
+// Raises a kernel's dynamic shared memory limit, once per kernel and context (again after a call from another context
+// of the device).
 template <auto KERNEL>
 struct Kernel {};
 template <auto KERNEL>
-cudaError_t allow_smem(Kernel<KERNEL>, int device, uint32_t bytes) {
-	static_assert(MAX_DEVICES <= 32);
-	static std::atomic<uint32_t> done{0};
-	uint32_t const bit = 1u << device;
-	if ((done.load(std::memory_order_acquire) & bit) != 0) return cudaSuccess;
+cudaError_t allow_smem(Kernel<KERNEL>, StreamScope const &on, uint32_t bytes) {
+	static std::atomic<uint64_t> raised_in[MAX_DEVICES];   // id of a context in which it has been raised; 0 = none
+	std::atomic<uint64_t> &last = raised_in[on.device];
+	if (last.load(std::memory_order_acquire) == on.state().id) return cudaSuccess;
 	cudaError_t const e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
-	if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+	if (e == cudaSuccess) last.store(on.state().id, std::memory_order_release);
 	return e;
 }
 
@@ -331,7 +354,7 @@ x17ai_DiagnosticBuffer *attn_launch(
 		plan.n_items = uint32_t(items);
 		dim3 grid(plan.n_items < sms ? plan.n_items : sms);
 		auto go = [&](auto kernel, uint32_t smem) -> cudaError_t {
-			cudaError_t const e2 = allow_smem(kernel, scope.device, smem);
+			cudaError_t const e2 = allow_smem(kernel, scope, smem);
 			if (e2 != cudaSuccess) return e2;
 			return launch(kernel, grid, x17::attn_stream_cfg::THREADS, smem, reinterpret_cast<cudaStream_t>(stream), dim3(NO_CLUSTER), tm_q, tm_kv, p, plan);
 		};
@@ -344,7 +367,7 @@ x17ai_DiagnosticBuffer *attn_launch(
 		auto go = [&](auto kernel, uint32_t smem) -> cudaError_t {
 			// at least 80 KB so that no more than two CTAs (2 x 256 TMEM columns) share an SM
 			smem = smem < 80u * 1024u ? 80u * 1024u : smem;
-			cudaError_t const e2 = allow_smem(kernel, scope.device, smem);
+			cudaError_t const e2 = allow_smem(kernel, scope, smem);
 			if (e2 != cudaSuccess) return e2;
 			return launch(kernel, grid, x17::attn_cfg::THREADS, smem, reinterpret_cast<cudaStream_t>(stream), dim3(NO_CLUSTER), tm_q, tm_kv, p);
 		};
@@ -509,7 +532,7 @@ cudaError_t gemm_go_pair_kind(StreamScope const &on, cudaStream_t stream, CUtens
 							  x17::GemmParams const &p) {
 	uint32_t const smem = x17::gemm_cfg::PAIR_SMEM_BYTES;
 	auto const kernel = x17::gemm_pair_kernel<EPI, F8>;
-	cudaError_t const ce = allow_smem(Kernel<&x17::gemm_pair_kernel<EPI, F8>>{}, on.device, smem);
+	cudaError_t const ce = allow_smem(Kernel<&x17::gemm_pair_kernel<EPI, F8>>{}, on, smem);
 	if (ce != cudaSuccess) return ce;
 	uint32_t const tiles = ((p.m + 2 * x17::gemm_cfg::BM - 1) / (2 * x17::gemm_cfg::BM)) * p.tiles_n;
 	uint32_t const fit = max_pair_clusters(kernel, smem, on.state().sm_count);
@@ -588,7 +611,7 @@ cudaError_t gemm_go_split_kind(StreamScope const &on, SplitPlan const &plan, cud
 							   x17::GemmParams const &p) {
 	using namespace x17::gemm_cfg;
 	constexpr Kernel<&x17::gemm_split_kernel<EPI, F8>> kernel{};
-	cudaError_t const ce = allow_smem(kernel, on.device, split_smem_bytes(BM, SPLIT_MAX_STAGES));
+	cudaError_t const ce = allow_smem(kernel, on, split_smem_bytes(BM, SPLIT_MAX_STAGES));
 	if (ce != cudaSuccess) return ce;
 	return launch(kernel, dim3(plan.grid), THREADS, plan.smem, stream, dim3(plan.sp.split), ta, tb, p, plan.sp);
 }
@@ -633,7 +656,7 @@ template <int EPI, bool F8>
 cudaError_t gemm_go_rows_kind(StreamScope const &on, RowsPlan const &plan, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tw,
 							  x17::GemmParams const &p) {
 	constexpr Kernel<&x17::gemm_rows_kernel<EPI, F8>> kernel{};
-	cudaError_t const ce = allow_smem(kernel, on.device, 112 * 1024);
+	cudaError_t const ce = allow_smem(kernel, on, 112 * 1024);
 	if (ce != cudaSuccess) return ce;
 	return launch(kernel, dim3(plan.grid), x17::rows_cfg::THREADS, plan.smem, stream, dim3(plan.rp.split), ta, tw, p, plan.rp);
 }
@@ -647,7 +670,7 @@ template <int EPI, bool F8>
 cudaError_t gemm_go_kind(StreamScope const &on, dim3 grid, cudaStream_t stream, CUtensorMap const &ta, CUtensorMap const &tb,
 						 x17::GemmParams const &p) {
 	uint32_t const smem = x17::gemm_cfg::SMEM_BYTES;
-	cudaError_t const ce = allow_smem(Kernel<&x17::gemm_kernel<EPI, F8>>{}, on.device, smem);
+	cudaError_t const ce = allow_smem(Kernel<&x17::gemm_kernel<EPI, F8>>{}, on, smem);
 	if (ce != cudaSuccess) return ce;
 	return launch(Kernel<&x17::gemm_kernel<EPI, F8>>{}, grid, x17::gemm_cfg::THREADS, smem, stream, dim3(NO_CLUSTER), ta, tb, p);
 }
@@ -775,8 +798,8 @@ static __device__ __align__(256) float g_noalloc_scratch[NOALLOC_SCRATCH_FLOATS]
 
 struct NoAllocDevice {
 	std::mutex mutex;
-	bool ready = false;        // set once the set-up has succeeded; a failed set-up is tried again by the next call
-	float *scratch = nullptr;  // device address of g_noalloc_scratch on this device
+	uint64_t context = 0;      // id of the context that the rest belongs to; a failed set-up is tried again by the next call
+	float *scratch = nullptr;  // device address of g_noalloc_scratch in that context
 	int sm_count = 0;
 };
 NoAllocDevice g_noalloc_dev[MAX_DEVICES];
@@ -1189,13 +1212,19 @@ x17ai_DiagnosticBuffer *x17ai_b200_attn_decode_i8_noalloc(
 		return make_diag("x17ai_b200: cannot resolve the device", who, ": cannot resolve the device");
 	}
 	NoAllocDevice &nd = g_noalloc_dev[int(dev)];
-	// First call on this device (with the device current): resolve the device address of the
-	// scratch array. In host code the array's name is only a stand-in, not a device pointer.
+	unsigned long long ctx_id = 0;
+	if (DRV(cuCtxGetId)(ctx, &ctx_id) != CUDA_SUCCESS) {
+		return make_diag("x17ai_b200: cannot enter the stream's context", who, ": the stream's context has no id");
+	}
+	// First call in this context (which is current): resolve the device address of the scratch array there. In host
+	// code the array's name is only a stand-in, not a device pointer.
 	// Only a successful set-up is remembered: after a failure (a first call made inside a stream capture, a
 	// transient error) the next call tries again.
+	float *scratch = nullptr;
+	int sm_count = 0;
 	{
 		std::lock_guard<std::mutex> lock(nd.mutex);
-		if (!nd.ready) {
+		if (nd.context != ctx_id) {
 			int major = 0;
 			cudaError_t e = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, int(dev));
 			if (e == cudaSuccess && major != 10) {
@@ -1212,12 +1241,14 @@ x17ai_DiagnosticBuffer *x17ai_b200_attn_decode_i8_noalloc(
 			}
 			nd.scratch = ptr;
 			nd.sm_count = sms;
-			nd.ready = true;
+			nd.context = ctx_id;
 		}
+		scratch = nd.scratch;
+		sm_count = nd.sm_count;
 	}
 	cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
 	size_t const pairs = batch * cfg->n_heads;
-	if (n_splits == 0) n_splits = choose_splits(pairs, kv_len, nd.sm_count);
+	if (n_splits == 0) n_splits = choose_splits(pairs, kv_len, sm_count);
 	uint32_t const d = uint32_t(cfg->head_dim);
 	size_t const need = n_splits > 1 ? pairs * n_splits * (d + 2) : 0;
 	if (n_splits > 65535 || need > NOALLOC_SCRATCH_FLOATS) {
@@ -1227,7 +1258,7 @@ x17ai_DiagnosticBuffer *x17ai_b200_attn_decode_i8_noalloc(
 	}
 	x17::DecodeParams p = decode_params(cfg, q, kv_cache, kv_capacity, kv_len, kv_lens, sink_k, sink_v, attn_temperature, out,
 										l, window_size, n_splits);
-	if (!decode_in_cluster(n_splits)) p.scratch = nd.scratch;  // every split writes its whole slot before the merge reads it
+	if (!decode_in_cluster(n_splits)) p.scratch = scratch;  // every split writes its whole slot before the merge reads it
 	return decode_go(who, s, cfg->head_dim, batch, p);
 }
 

@@ -20,6 +20,7 @@
 	X(cuCtxPopCurrent)            \
 	X(cuCtxGetDevice)             \
 	X(cuCtxGetCurrent)            \
+	X(cuCtxGetId)                 \
 	X(cuStreamCreate)             \
 	X(cuStreamDestroy)            \
 	X(cuStreamSynchronize)        \
