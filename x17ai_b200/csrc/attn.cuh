@@ -91,13 +91,23 @@ X17_DEV u32 seen_columns(u32 col0, u32 lo, u32 span) {
 	return below(lo + span) & ~below(lo);
 }
 
+// The row maximum m of x = t * a. To nearest: rounded up, all of a row's x = fma(t, a, -m) move by up to an ulp of m (1 to 2 %
+// more error against 64 bits in the scaled mode where the scores are large). The largest x may then be half an ulp of m
+// above zero: below |m| = 2^16 that leaves rint(255 * 2^x) at 255, from there on m is rounded up instead (rint would
+// reach 256, no byte).
+X17_DEV f32 largest_score(f32 t, f32 a) {
+	f32 const m = __fmul_rn(t, a);
+	return fabsf(m) < 65536.0f ? m : __fmul_ru(t, a);
+}
+
 // N score columns of one row -> probabilities: accumulates the un-rounded exp2 into sum[4] and
 // returns rint(255 * p) packed four to a word. EDGE: only columns lo <= col < lo + span are visible.
 // The four f32 operations per element are issued as packed f32x2 instructions (two elements per
 // issue slot); int -> float is one I2FP. float -> u8: p times the subnormal 255 * 2^-149 is rounded to a whole number of
 // 2^-149, which is rint(255 p) as the bits of the word (the same rounding of the same exact product as adding 1.5 * 2^23),
 // and since the words are plain small numbers one packed fma by 2^16 puts two of four bytes in place, where the
-// 1.5 * 2^23 trick needs three byte permutes. Subnormal operands cost the packed instructions nothing.
+// 1.5 * 2^23 trick needs three byte permutes. (That wants bytes: a word of 256 in the upper place would change the lower
+// one; see largest_score.) Subnormal operands cost the packed instructions nothing.
 // Together with the bit masks above: 8 x 32 heads x 8192 x 128, window 1024 1141 -> 1095 us, 2 x 64 x 8192 x 64 522 -> 500,
 // 2 x 64 x 2000 x 32, window 512 85.1 -> 80.7, 64 x 16384 x 32 without a window 3165 -> 3134.
 // FP8: P is written as OCP e4m3 of 256 * p instead of u8 of 255 * p.
@@ -186,14 +196,6 @@ X17_DEV void extreme_chunk(u32 const (&r)[32], u32 col0, u32 lo, u32 span, i32 (
 // single loads with a test per key) 810 -> 472 us; 2 x 64 x 8192 x 64, no window 3.85 -> 2.88 ms. What is left above the
 // FixedI8 kernel (1.14 ms) is issue slots: 2 instructions per score against 0.4 in the first sweep, 5.8 against 4.2 in the second.
 constexpr u32 FRAG_ROWS = 4;   // rows of a thread's score fragment
-
-// The row maximum m, to nearest as every mode has it (rounded up, all of a row's x move by up to an ulp of m, and 1 to 2 %
-// more error against 64 bits comes out where the scores are large). The largest x = fma(t, a, -m) may then be half an ulp
-// of m above zero: below |m| = 2^16 that leaves rint(255 * 2^x) at 255, from there on m is rounded up instead.
-X17_DEV f32 largest_score(f32 t, f32 a) {
-	f32 const m = __fmul_rn(t, a);
-	return fabsf(m) < 65536.0f ? m : __fmul_ru(t, a);
-}
 X17_DEV u32 frag_row(u32 slot, u32 lane) { return 8 * slot + lane / 4; }   // inside the warp's 32 rows
 
 // N column pairs' scales: keys key + 8 j + {0, 1}. IN_PAIRS: `sc + key` is 8-byte aligned and every key exists.
@@ -646,7 +648,7 @@ X17_DEV void attn_fwd_body(CUtensorMap const *tm_q_ptr, CUtensorMap const *tm_kv
 		{
 			i32 const e = pos_t ? max(max(ext[0], ext[1]), max(ext[2], ext[3]))
 								: min(min(ext[0], ext[1]), min(ext[2], ext[3]));
-			if (e != (pos_t ? INT32_MIN : INT32_MAX)) cand = __fmul_rn(__int2float_rn(e), temp);
+			if (e != (pos_t ? INT32_MIN : INT32_MAX)) cand = largest_score(__int2float_rn(e), temp);
 		}
 		// per-token-scale mode: [half][row] extremes and value scales, then [row] (a_row, -m, 255 / g), in the P buffer,
 		// which nothing uses before the second sweep

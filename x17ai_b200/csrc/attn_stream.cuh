@@ -574,7 +574,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
 						f32 cand = -INFINITY;
 						i32 const e = pos_t ? max(max(ext[0], ext[1]), max(ext[2], ext[3]))
 											: min(min(ext[0], ext[1]), min(ext[2], ext[3]));
-						if (a.s1 && e != (pos_t ? INT32_MIN : INT32_MAX)) cand = __fmul_rn(__int2float_rn(e), temp1);
+						if (a.s1 && e != (pos_t ? INT32_MIN : INT32_MAX)) cand = largest_score(__int2float_rn(e), temp1);
 						f32 const part = __fadd_rn(__fadd_rn(sum[0], sum[1]), __fadd_rn(sum[2], sum[3]));
 						xc[(0 * 4 + cq) * BQ + row] = __float_as_uint(cand);
 						xc[(1 * 4 + cq) * BQ + row] = __float_as_uint(part);
