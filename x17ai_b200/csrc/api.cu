@@ -547,10 +547,19 @@ cudaError_t gemm_go_pair(bool f8, StreamScope const &on, cudaStream_t stream, CU
 			  : gemm_go_pair_kind<EPI, false>(on, stream, ta, tb_half, p);
 }
 
-// The form for few rows (gemm.cuh): a cluster of up to four CTAs shares one 128 x 256 tile, K split over it.
-// Taken (default tiling only) for up to 128 rows, where a persistent form has one CTA per column tile at most, and
-// for more rows while the CTA-pair form's tiles would keep no more than half of the SMs busy and K is long enough
-// (4096) to pay for the exchange of the parts.
+// The split form (gemm.cuh): a cluster of up to four CTAs shares one 128 x 256 tile, K split over it. Default tiling only.
+// Where the line lies (int8 and e4m3, plain and per-head epilogues, weights cold; time over the persistent form's):
+//   up to 128 rows (those that gemm_rows.cuh does not take): a persistent form has one CTA per column tile at most.
+//   - More tiles than SMs: never. A second wave without the overlap of epilogue and main loop costs 7 to 66 %
+//     (49 to 128 rows, N 40960 to 131072).
+//   - Tiles for more than half of the SMs, so K stays whole: up to 16 K blocks 0.91 to 0.98, beyond 0.96 to 1.04.
+//   - Otherwise K has to be long enough to pay for the exchange of the parts, the longer the more rows there are to
+//     exchange: int8 at 64 rows 1.1 to 1.2 with 4 blocks, 0.95 to 1.06 with 8, 0.73 to 0.89 with 16; at 128 rows 1.1 to 1.3
+//     with 8, 0.9 to 1.03 with 16; e4m3 (a slower MMA to hide it under) 0.81 to 0.94 at 64 rows and 1.0 to 1.1 at 128 with 8.
+//   - Tiles of heads, which one CTA finishes: 0.9 to 1.0 from 8 blocks on at 32 tiles, from 16 on at 8 (0.84 to 1.05), below
+//     from 32 on (0.57 to 1.13).
+//   more rows, while the CTA-pair form's tiles keep no more than half of the SMs busy: 32 blocks (0.65 to 0.96), heads of width
+//   128 64 (0.75 to 0.95; 1.03 to 1.15 with 32).
 struct SplitPlan {
 	x17::SplitParams sp{};
 	uint32_t grid = 0, smem = 0;
@@ -577,14 +586,21 @@ uint32_t deal_chunks(x17::SplitParams &sp, uint32_t head_dim) {
 	}
 	return most;
 }
-SplitPlan plan_split(size_t rows, size_t n_raw, size_t k, uint32_t head_dim, int sm_count) {
+SplitPlan plan_split(size_t rows, size_t n_raw, size_t k, bool f8, uint32_t head_dim, int sm_count) {
 	using namespace x17::gemm_cfg;
 	SplitPlan plan;
 	if (g_gemm_tiling.load(std::memory_order_relaxed) != X17AI_B200_GEMM_AUTO) return plan;
 	size_t const tiles_n = (n_raw + BN - 1) / BN, pair_tiles = ((rows + 2 * BM - 1) / (2 * BM)) * tiles_n;
 	size_t const tiles_m = (rows + BM - 1) / BM, tiles = tiles_m * tiles_n, k_blocks = k / BK;
-	if (rows > BM && (4 * pair_tiles > size_t(sm_count) || k_blocks < 32)) return plan;
-	if (tiles > (size_t(1) << 27)) return plan;
+	if (rows > BM) {
+		if (4 * pair_tiles > size_t(sm_count) || k_blocks < (head_dim == 128 ? 64u : 32u)) return plan;
+	} else if (2 * tiles > size_t(sm_count)) {
+		if (tiles > size_t(sm_count) || k_blocks > 16) return plan;
+	} else if (head_dim != 0) {
+		if (k_blocks < (tiles >= 32 ? 8u : tiles >= 8 ? 16u : 32u)) return plan;
+	} else if (k_blocks < 8 || k_blocks * (f8 ? 14 : 8) < rows) {
+		return plan;
+	}
 	x17::SplitParams &sp = plan.sp;
 	sp.tiles_m = uint32_t(tiles_m);
 	sp.a_rows = rows >= BM ? BM : uint32_t((rows + 7) / 8 * 8);
@@ -625,17 +641,24 @@ cudaError_t gemm_go_split(bool f8, StreamScope const &on, SplitPlan const &plan,
 // costs more than the 256-column tiles of the split form save: at 64 rows the e4m3 x int8 projection of
 // [8192, 2 x 14336] takes 54 us against 45). K is split over a cluster of up to four CTAs as long as all CTAs run at
 // once, two to an SM, and each has four K blocks or more.
+// Above 32 rows (48 MMA columns) some calls are left to the other forms: tiles of heads with K under 32 blocks (a row's sum
+// of squares is one thread's: 1.02 to 1.25 of the persistent form's time with 8 and 16 blocks, 0.66 to 0.98 with 32), more
+// than two rounds of tiles with K under 12 blocks (1.05 to 1.17), and e4m3 from the second round on with up to 16 blocks
+// (0.93 to 1.14).
 struct RowsPlan {
 	x17::RowsParams rp{};
 	uint32_t grid = 0, smem = 0;
 	explicit operator bool() const { return grid != 0; }
 };
-RowsPlan plan_rows(size_t rows, size_t n_raw, size_t k, bool heads, int sm_count) {
+RowsPlan plan_rows(size_t rows, size_t n_raw, size_t k, bool f8, bool heads, int sm_count) {
 	using namespace x17::rows_cfg;
 	RowsPlan plan;
 	if (g_gemm_tiling.load(std::memory_order_relaxed) != X17AI_B200_GEMM_AUTO || rows > MAX_TOK) return plan;
 	size_t const tiles = n_raw / WM, k_blocks = k / BK;
-	if (tiles > (size_t(1) << 27)) return plan;
+	if (rows > 32) {
+		size_t const at_once = 2 * size_t(sm_count);
+		if ((heads && k_blocks < 32) || (tiles > 2 * at_once && k_blocks < 12) || (f8 && tiles > at_once && k_blocks <= 16)) return plan;
+	}
 	x17::RowsParams &rp = plan.rp;
 	rp.a_box = uint32_t((rows + 7) / 8 * 8);
 	rp.n_tok = uint32_t((rows + 15) / 16 * 16);
@@ -1305,10 +1328,11 @@ x17ai_DiagnosticBuffer *x17ai_b200_gemm_fwd(
 	size_t const k_a = cfg->a_cols;
 	size_t const k_total = plan.split ? 2 * k_a : k_a;
 	CUtensorMap ta, tb;
-	RowsPlan const few = plan_rows(a_rows, cfg->b_rows, k_total, plan.epi == x17::EPI_L2NORM_KV, scope.state().sm_count);
-	SplitPlan const split = plan_split(a_rows, cfg->b_rows, k_total, plan.epi == x17::EPI_L2NORM_KV ? uint32_t(cfg->head_dim) : 0u,
-									   scope.state().sm_count);
-	bool const pair = !split && g_gemm_tiling.load(std::memory_order_relaxed) != X17AI_B200_GEMM_ONE_CTA && a_rows > BM
+	RowsPlan const few = plan_rows(a_rows, cfg->b_rows, k_total, plan.f8, plan.epi == x17::EPI_L2NORM_KV, scope.state().sm_count);
+	SplitPlan const split = few ? SplitPlan{}
+								: plan_split(a_rows, cfg->b_rows, k_total, plan.f8,
+											 plan.epi == x17::EPI_L2NORM_KV ? uint32_t(cfg->head_dim) : 0u, scope.state().sm_count);
+	bool const pair = !few && !split && g_gemm_tiling.load(std::memory_order_relaxed) != X17AI_B200_GEMM_ONE_CTA && a_rows > BM
 					  && cfg->b_rows % BN == 0 && scope.state().sm_count >= 2;
 	CUresult e = make_map_2d(&ta, a, k_a, a_rows, k_a, BK, few ? few.rp.a_box : split ? split.sp.a_rows : BM);
 	if (e == CUDA_SUCCESS) e = make_map_2d(&tb, b, k_total, cfg->b_rows, k_total, BK, few || pair ? BN / 2 : BN);
@@ -1380,9 +1404,9 @@ x17ai_DiagnosticBuffer *x17ai_b200_qkvg_fwd_i8(
 	using namespace x17::gemm_cfg;
 	size_t const n_raw = n_q + n_kv + n_g;
 	CUtensorMap ta, tb;
-	RowsPlan const few = plan_rows(rows, n_raw, cfg->model_dim, true, scope.state().sm_count);
-	SplitPlan const split = plan_split(rows, n_raw, cfg->model_dim, uint32_t(cfg->head_dim), scope.state().sm_count);
-	bool const pair = !split && g_gemm_tiling.load(std::memory_order_relaxed) != X17AI_B200_GEMM_ONE_CTA && rows > BM
+	RowsPlan const few = plan_rows(rows, n_raw, cfg->model_dim, false, true, scope.state().sm_count);
+	SplitPlan const split = few ? SplitPlan{} : plan_split(rows, n_raw, cfg->model_dim, false, uint32_t(cfg->head_dim), scope.state().sm_count);
+	bool const pair = !few && !split && g_gemm_tiling.load(std::memory_order_relaxed) != X17AI_B200_GEMM_ONE_CTA && rows > BM
 					  && n_raw % BN == 0 && scope.state().sm_count >= 2;
 	CUresult e = make_map_2d(&ta, x, cfg->model_dim, rows, cfg->model_dim, BK, few ? few.rp.a_box : split ? split.sp.a_rows : BM);
 	if (e == CUDA_SUCCESS) e = make_map_2d(&tb, w_qkvg, cfg->model_dim, n_raw, cfg->model_dim, BK, few || pair ? BN / 2 : BN);
