@@ -10,12 +10,12 @@ from oracle import formats, gemm as o_gemm
 pytestmark = pytest.mark.gpu
 
 
-@pytest.fixture(autouse=True, params=["one_cta", "cta_pair"])
+@pytest.fixture(autouse=True, params=["one_cta", "cta_pair", "auto"])
 def gemm_tiling(request):
-    """Every test runs with both tilings of the GEMM: one CTA per 128 x 256 tile, and clusters of two CTAs on
-    256 x 256 tiles (taken for inputs of more than 128 rows whose N is a multiple of 256)."""
+    """Every test runs with every tiling of the GEMM: one CTA per 128 x 256 tile, clusters of two CTAs on
+    256 x 256 tiles (taken for inputs of more than 128 rows whose N is a multiple of 256), and the default, chosen per launch."""
     from x17ai_b200 import kernels as K
-    K.set_gemm_tiling(K.GEMM_CTA_PAIR if request.param == "cta_pair" else K.GEMM_ONE_CTA)
+    K.set_gemm_tiling({"one_cta": K.GEMM_ONE_CTA, "cta_pair": K.GEMM_CTA_PAIR, "auto": K.GEMM_AUTO}[request.param])
     yield request.param
     K.set_gemm_tiling()
 
