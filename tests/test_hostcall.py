@@ -1,5 +1,5 @@
-"""The native launch path (csrc/hostcall.cpp) on arguments whose attributes cannot be read: the launchers raise, as their Python
-checks do, and the process goes on."""
+"""The native launch path (csrc/hostcall.cpp): on arguments whose attributes cannot be read the launchers raise, as their Python
+checks do, and the process goes on; without it they launch through those checks."""
 import subprocess
 import sys
 from pathlib import Path
@@ -59,3 +59,38 @@ def test_sparse_tensors_raise(stream):
     x = torch.ones((4, 512), dtype=torch.uint8).to_sparse_csr().cuda()
     with pytest.raises(RuntimeError):
         K.rms_norm(stream, K.RMS_E4M3_FIXED, x, torch.zeros((4, 512), dtype=torch.int8, device="cuda"))
+
+
+@pytest.fixture(params=["missing", "another torch"])
+def no_native_path(request, monkeypatch):
+    import types
+    import x17ai_b200
+    from x17ai_b200 import _lib
+    mod = types.SimpleNamespace(built_for="torch 0.1;") if request.param == "another torch" else None
+    monkeypatch.setattr(_lib, "_hostcall", None)
+    monkeypatch.setitem(sys.modules, "x17ai_b200._hostcall", mod)
+    monkeypatch.delattr(x17ai_b200, "_hostcall", raising=False)
+    if mod is not None:
+        monkeypatch.setattr(x17ai_b200, "_hostcall", mod, raising=False)
+
+
+def test_kernels_without_the_native_path(no_native_path):
+    from x17ai_b200 import X17Error, kernels as K
+    with pytest.warns(RuntimeWarning, match="native launch path"):
+        kern = K.GemmKernel(K.attn_q_fwd_config(128, 128))
+    t = torch.zeros((16, 64), dtype=torch.int8)
+    with pytest.raises(X17Error, match="64 columns, but should have 128"):
+        kern.launch(type("Stream", (), {"handle": 1})(), t, t, t)
+
+
+@pytest.mark.gpu
+def test_launches_without_the_native_path(stream, no_native_path):
+    from x17ai_b200 import kernels as K
+    x = torch.randn(16, 512, device="cuda").to(torch.bfloat16)
+    outs = [torch.zeros((16, 512), dtype=torch.int8, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    with pytest.warns(RuntimeWarning, match="native launch path"):
+        K.rms_norm(stream, K.RMS_BF16_FIXED, x, outs[0])
+    K.rms_norm(stream, K.RMS_BF16_FIXED, x, outs[1])
+    stream.synchronize()
+    assert outs[0].any() and torch.equal(*outs)

@@ -347,4 +347,9 @@ PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_hostcall", nullptr, -1, metho
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__hostcall() { return PyModule_Create(&module_def); }
+PyMODINIT_FUNC PyInit__hostcall() {
+	PyObject *m = PyModule_Create(&module_def);
+	// the version of torch whose objects this reads
+	if (m != nullptr && PyModule_AddStringConstant(m, "built_for", X17_BUILT_FOR) != 0) Py_CLEAR(m);
+	return m;
+}
