@@ -94,3 +94,20 @@ def test_launches_without_the_native_path(stream, no_native_path):
     K.rms_norm(stream, K.RMS_BF16_FIXED, x, outs[1])
     stream.synchronize()
     assert outs[0].any() and torch.equal(*outs)
+
+
+@pytest.mark.gpu
+def test_a_replaced_config_is_the_one_that_launches(stream):
+    from x17ai_b200 import X17Error, kernels as K
+    x, w = (torch.randint(-9, 9, s, dtype=torch.int8, device="cuda") for s in ((16, 128), (256, 128)))
+    outs = [torch.zeros((16, 256), dtype=torch.int8, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    kern = K.GemmKernel(K.attn_q_fwd_config(128, 128))
+    kern.config = K.attn_q_fwd_config(128, 256)
+    kern.launch(stream, x, w, outs[0])
+    K.GemmKernel(K.attn_q_fwd_config(128, 256)).launch(stream, x, w, outs[1])
+    stream.synchronize()
+    assert outs[0].any() and torch.equal(*outs)
+    with pytest.raises(X17Error, match="256 rows, but should have 128"):
+        kern.config = K.attn_q_fwd_config(128, 128)
+        kern.launch(stream, x, w, outs[0])

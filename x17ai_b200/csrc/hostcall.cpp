@@ -240,7 +240,7 @@ PyObject *gemm(PyObject *, PyObject *const *v, Py_ssize_t n) {
 	if (!a.is2(ANY, k, g->a_dtype) || !b.is2(rows, split ? 2 * k : k, split ? int32_t(X17AI_DTYPE_E4M3) : g->b_dtype)) Py_RETURN_FALSE;
 	int64_t const m = a.t->size(0);
 	if (!c.is2(m, whole ? rows : rows / 2, g->c_dtype)) Py_RETURN_FALSE;
-	if (g->epilogue == X17AI_EPILOGUE_RMS_NORM && (rr.none() || !rr.is2(m, rows / (2 * int64_t(g->head_dim)), F32))) Py_RETURN_FALSE;
+	if (g->epilogue == X17AI_EPILOGUE_RMS_NORM && (g->head_dim == 0 || rr.none() || !rr.is2(m, rows / (2 * int64_t(g->head_dim)), F32))) Py_RETURN_FALSE;
 	if (g->epilogue == X17AI_EPILOGUE_RESIDUAL && (res.none() || !res.is2(m, rows / 2, I8))) Py_RETURN_FALSE;
 	return launch([&] {
 		return p_x17ai_b200_gemm_fwd(stream, g, a.ptr(), size_t(m), b.ptr(), g->b_rows, c.ptr(), (float *)rr.ptr(),

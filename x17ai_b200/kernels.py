@@ -122,7 +122,20 @@ class AttnKernelConfig:
         return _lib.AttnConfig(self.n_heads, self.head_dim, self.q_stride, self.kv_stride, self.o_stride)
 
 
-class AttnKernel:
+class _Configured:
+    """`config` and its C form, which the native launches read by address. Assigning `config` replaces both."""
+
+    @property
+    def config(self):
+        return self._c_config[0]
+
+    @config.setter
+    def config(self, config):
+        c = config._c()
+        self._c_config = (config, c, ctypes.addressof(c))
+
+
+class AttnKernel(_Configured):
     """AttnKernel::new + launch (attn.rs:171-232, 353-447). `q`, `kv`, `out` may carry a leading
     batch dimension ([B, S, cols]); the reference's 2-D call is batch 1."""
 
@@ -131,8 +144,7 @@ class AttnKernel:
         self._lib = _lib.load()
         self._native = _lib.hostcall()
         meta = _lib.AttnMeta()
-        cfg = self._cfg = config._c()
-        self._cfg_addr = ctypes.addressof(cfg)
+        cfg = self._c_config[1]
         check(self._lib.x17ai_b200_attn_meta(ctypes.byref(cfg), ctypes.byref(meta)))
         self.THREADS_PER_BLOCK = int(meta.threads_per_block)
         self.SMEM_BYTES = int(meta.smem_bytes)
@@ -163,7 +175,8 @@ class AttnKernel:
         return batch, seq_len
 
     def launch(self, stream, q, kv, sink_k, sink_v, attn_temperature, out, l=None, window_size=0):
-        if _launched(self._native.attn(self._cfg_addr, stream.handle, q, kv, sink_k, sink_v, attn_temperature, out, l, window_size)):
+        held = self._c_config   # the C form lives as long as the call
+        if _launched(self._native.attn(held[2], stream.handle, q, kv, sink_k, sink_v, attn_temperature, out, l, window_size)):
             return
         batch, seq_len = self._shapes(q, kv, sink_k, sink_v, attn_temperature, out, l)
         cfg = self.config._c()
@@ -245,7 +258,8 @@ class AttnKernel:
 
     def launch_pv_fp8(self, stream, q, kv, sink_k, sink_v, attn_temperature, v_scale, out, l=None, window_size=0):
         """fp8 P.V variant: kv holds int8 K and e4m3 V bytes (int8 view), sink_v e4m3, out bf16."""
-        if _launched(self._native.attn_pv_fp8(self._cfg_addr, stream.handle, q, kv, sink_k, sink_v, attn_temperature, v_scale, out, l,
+        held = self._c_config   # the C form lives as long as the call
+        if _launched(self._native.attn_pv_fp8(held[2], stream.handle, q, kv, sink_k, sink_v, attn_temperature, v_scale, out, l,
                                               window_size)):
             return
         c = self.config
@@ -267,7 +281,8 @@ class AttnKernel:
                       window_size=0):
         """Inputs with one f32 scale per token and head (value = scale * code; `q_scale`, `k_scale`, `v_scale`
         f32 [B, H, S] or [H, S]), bf16 output: x17ai_b200_attn_fwd_i8_scaled."""
-        if _launched(self._native.attn_scaled(self._cfg_addr, stream.handle, q, q_scale, kv, k_scale, v_scale, sink_k, sink_v,
+        held = self._c_config   # the C form lives as long as the call
+        if _launched(self._native.attn_scaled(held[2], stream.handle, q, q_scale, kv, k_scale, v_scale, sink_k, sink_v,
                                               attn_temperature, out, l, window_size)):
             return
         c = self.config
@@ -305,7 +320,8 @@ class AttnKernel:
         """One new token per sequence: q [B, q_stride], kv_cache [B, T, kv_stride], out [B, o_stride].
         `no_alloc=True` takes the entry point that keeps its split-KV partials in the library's built-in
         4 MiB scratch instead of allocating (see x17ai_b200_attn_decode_i8_noalloc in the header)."""
-        if _launched(self._native.decode(self._cfg_addr, stream.handle, q, kv_cache, kv_len, sink_k, sink_v, attn_temperature, out, l,
+        held = self._c_config   # the C form lives as long as the call
+        if _launched(self._native.decode(held[2], stream.handle, q, kv_cache, kv_len, sink_k, sink_v, attn_temperature, out, l,
                                          window_size, kv_lens, n_splits, no_alloc)):
             return
         c = self.config
@@ -356,7 +372,7 @@ class GemmConfig:
                                self.inp_scale, self.out_scale, self.eps, self.head_dim)
 
 
-class GemmKernel:
+class GemmKernel(_Configured):
     """GemmKernel<E>::new + launch (gemm.rs:368-443, 591-641)."""
 
     def __init__(self, config: GemmConfig):
@@ -364,8 +380,7 @@ class GemmKernel:
         self._lib = _lib.load()
         self._native = _lib.hostcall()
         meta = _lib.GemmMeta()
-        cfg = self._cfg = config._c()
-        self._cfg_addr = ctypes.addressof(cfg)
+        cfg = self._c_config[1]
         check(self._lib.x17ai_b200_gemm_meta(ctypes.byref(cfg), ctypes.byref(meta)))
         self.THREADS_PER_BLOCK = int(meta.threads_per_block)
         self.SMEM_BYTES = int(meta.smem_bytes)
@@ -373,7 +388,8 @@ class GemmKernel:
         self.N_PER_BLOCK = int(meta.n_per_block)
 
     def launch(self, stream, a, b, c, rrms=None, residual=None):
-        if _launched(self._native.gemm(self._cfg_addr, stream.handle, a, b, c, rrms, residual)):
+        held = self._c_config   # the C form lives as long as the call
+        if _launched(self._native.gemm(held[2], stream.handle, a, b, c, rrms, residual)):
             return
         g = self.config
         a_rows = self.check_shapes(a, b, c, rrms, residual)
