@@ -786,17 +786,21 @@ x17::DecodeParams decode_params(x17ai_AttnConfig const *cfg, int8_t const *q, in
 // Splits whose partials meet in a cluster's shared memory (the others need p.scratch).
 bool decode_in_cluster(size_t n_splits) { return n_splits <= x17::dec_cfg::MAX_CLUSTER_SPLITS; }
 
-template <uint32_t D>
-x17ai_DiagnosticBuffer *decode_go_dim(char const *who, cudaStream_t s, size_t batch, x17::DecodeParams const &p) {
+template <uint32_t D, bool AHEAD>
+x17ai_DiagnosticBuffer *decode_go_kind(char const *who, cudaStream_t s, size_t batch, x17::DecodeParams const &p) {
 	using namespace x17::dec_cfg;
-	constexpr Kernel<&x17::attn_decode_kernel<D>> kernel{};
 	cudaError_t ce;
 	bool merge = false;
 	if (p.n_splits > 1 && p.scratch == nullptr) {
-		uint32_t const z = p.n_splits < MAX_CLUSTER ? p.n_splits : MAX_CLUSTER;
-		ce = launch(kernel, dim3(p.n_heads, unsigned(batch), z), THREADS, partials_bytes<D>(p.n_splits), s, dim3(1, 1, z), p);
+		// The same number of splits for every CTA, give or take one: ten splits on eight CTAs take as long as on five, and
+		// their cluster needs eight free places (4 x 32 heads x 16384 keys, width 128 121 -> 98 us; splits of different
+		// lengths before the launch 100).
+		uint32_t const each = (p.n_splits + MAX_CLUSTER - 1) / MAX_CLUSTER, z = (p.n_splits + each - 1) / each;
+		ce = launch(Kernel<&x17::attn_decode_kernel<D, true, AHEAD>>{}, dim3(p.n_heads, unsigned(batch), z), THREADS,
+					partials_bytes<D>(p.n_splits), s, dim3(1, 1, z), p);
 	} else {
-		ce = launch(kernel, dim3(p.n_heads, unsigned(batch), p.n_splits), THREADS, 0, s, dim3(NO_CLUSTER), p);
+		ce = launch(Kernel<&x17::attn_decode_kernel<D, false, AHEAD>>{}, dim3(p.n_heads, unsigned(batch), p.n_splits), THREADS, 0, s,
+					dim3(NO_CLUSTER), p);
 		merge = p.n_splits > 1;
 		if (ce == cudaSuccess && merge) {
 			ce = launch(Kernel<&x17::attn_decode_merge_kernel<D>>{}, dim3(p.n_heads, unsigned(batch)), D, 0, s, dim3(NO_CLUSTER), p);
@@ -806,6 +810,12 @@ x17ai_DiagnosticBuffer *decode_go_dim(char const *who, cudaStream_t s, size_t ba
 	x17ai_DiagnosticBuffer *res = launch_result(who);
 	if (res == nullptr && merge) g_launches.fetch_add(1, std::memory_order_relaxed);
 	return res;
+}
+template <uint32_t D>
+x17ai_DiagnosticBuffer *decode_go_dim(char const *who, cudaStream_t s, size_t batch, x17::DecodeParams const &p) {
+	uint32_t const longest = p.kv_lens != nullptr ? p.kv_capacity : p.kv_len;   // (the lengths themselves are on the device)
+	uint32_t const keys = longest < p.window ? longest : p.window;
+	return keys / p.n_splits > 2 * x17::DECODE_STEP<D> ? decode_go_kind<D, true>(who, s, batch, p) : decode_go_kind<D, false>(who, s, batch, p);
 }
 x17ai_DiagnosticBuffer *decode_go(char const *who, cudaStream_t s, size_t head_dim, size_t batch, x17::DecodeParams const &p) {
 	return head_dim == 128 ? decode_go_dim<128>(who, s, batch, p)

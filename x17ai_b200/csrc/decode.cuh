@@ -10,8 +10,8 @@
 // (16 bytes per lane, 32 / (D/16) rows per warp instruction): q.k with dp4a + a butterfly
 // inside the group, online softmax per group with lazy rescale (the int32 P.V accumulators
 // are only flushed to f32 when the group's running maximum moves), P.V with dp4a after a 4x4
-// byte transpose of four V rows. The loads of the next step are in flight under the arithmetic of the current one
-// (a split of 256 keys is two steps: without that its time is two DRAM latencies on top of the launch).
+// byte transpose of four V rows. From three steps on the loads of the next step are in flight under the arithmetic of the
+// current one.
 // Groups, warps and (with n_splits > 1) splits are merged with
 // the usual (max, sum, O) log-sum-exp combine; the sink token enters as one more partial.
 // The splits of a (head, batch) form a cluster of up to 8 CTAs (a CTA takes every 8th split where there are more);
@@ -112,14 +112,24 @@ X17_DEV void merge_partials(f32 const *src, u32 n, u32 d, f32 &fm, f32 &fs, f32 
 	}
 }
 
-// two CTAs per SM: 128 registers hold the rows in work and the rows on their way
+// Key rows that a CTA takes at once.
 template <u32 D>
+constexpr u32 DECODE_STEP = dec_cfg::WARPS * (512 / D) * dec_cfg::UNROLL;
+
+// Two CTAs per SM: 128 registers hold the rows in work and the rows on their way.
+// CLUSTER: the splits of a (sequence, head) form a cluster and meet in shared memory; otherwise a CTA is one split.
+// AHEAD: the next step's rows are loaded under the arithmetic of the current one: from three steps on (1639 keys a split at
+// width 64 62.5 -> 59.7 us, 863 at width 128 59.1 -> 57.0). With one or two steps there is little to load ahead, and what it
+// costs to hold the rows twice shows: 256 x 32 heads, 16 keys, 61.9 us without and 66.5 with it at width 32, 62.1 and 67.9
+// at 128; 128 x 8 heads, 512 keys in two splits, width 64 30.0 and 31.1.
+template <u32 D, bool CLUSTER, bool AHEAD>
 __global__ void __launch_bounds__(dec_cfg::THREADS, 2)
 attn_decode_kernel(const DecodeParams p) {
 	using namespace dec_cfg;
 	static_assert(D == 32 || D == 64 || D == 128);
 	constexpr u32 LPR = D / 16;        // lanes per key row
 	constexpr u32 RPI = 32 / LPR;      // key rows per warp instruction
+	static_assert(DECODE_STEP<D> == WARPS * RPI * UNROLL);
 	constexpr f32 NEG_BIG = -3.0e38f;
 
 	u32 const head = blockIdx.x;
@@ -129,7 +139,7 @@ attn_decode_kernel(const DecodeParams p) {
 	u32 const grp = lane / LPR;        // which row of the instruction this lane works on
 	u32 const sub = lane % LPR;        // which 16-byte chunk of the row
 
-	cluster_arrive();   // "this CTA runs" (a launch without clusters is one of single CTAs)
+	if constexpr (CLUSTER) cluster_arrive();   // "this CTA runs"
 	pdl_wait();
 	u32 const kv_len = p.kv_lens ? min(p.kv_lens[batch], p.kv_capacity) : p.kv_len;
 	u32 const w = p.window;
@@ -158,8 +168,8 @@ attn_decode_kernel(const DecodeParams p) {
 	f32 fm = 0.0f, fs = 0.0f, fo = 0.0f;   // of the CTA's split, in the threads below D
 	// Shared memory of another CTA may be written only once that CTA is known to run; being scheduled together is not enough,
 	// and a split without keys gets to its store within a few hundred cycles. (Asked for at entry: 5.51 -> 5.54 us a call for
-	// one sequence of 1500 keys. Behind a branch on the launch's form the loop spilled a register: 2 %.)
-	cluster_wait();
+	// one sequence of 1500 keys.)
+	if constexpr (CLUSTER) cluster_wait();
 	#pragma unroll 1
 	for (u32 split = blockIdx.z; split < p.n_splits; split += gridDim.z) {
 		u32 const s_lo = k_lo + split * per_split;
@@ -184,15 +194,19 @@ attn_decode_kernel(const DecodeParams p) {
 		u32 since_flush = 0;  // an int32 accumulator takes at most 4 * 255 * 127 per step: flush long before 2^31
 		u32 t0 = s_lo + (warp * UNROLL) * RPI;
 		uint4 kn[UNROLL], vn[UNROLL];
-		if (t0 < s_hi) load(t0, kn, vn);
+		if (AHEAD && t0 < s_hi) load(t0, kn, vn);
 		for (; t0 < s_hi; t0 += step) {
 			uint4 kq[UNROLL], vq[UNROLL];
+			if constexpr (AHEAD) {
 #pragma unroll
-			for (u32 u = 0; u < UNROLL; ++u) {
-				kq[u] = kn[u];
-				vq[u] = vn[u];
+				for (u32 u = 0; u < UNROLL; ++u) {
+					kq[u] = kn[u];
+					vq[u] = vn[u];
+				}
+				if (t0 + step < s_hi) load(t0 + step, kn, vn);
+			} else {
+				load(t0, kq, vq);
 			}
-			if (t0 + step < s_hi) load(t0 + step, kn, vn);
 			// ---- scores of UNROLL rows per group ----
 			bool valid[UNROLL];
 			f32 s[UNROLL];
@@ -282,32 +296,31 @@ attn_decode_kernel(const DecodeParams p) {
 				fo = __fmaf_rn(fo, a, sh_o[wq][d] * b);
 				fm = nm;
 			}
-			if (p.n_splits > 1) {
-				if (p.scratch != nullptr) {
-					f32 *dst = p.scratch + ((u64(batch) * p.n_heads + head) * p.n_splits + split) * (D + 2);
-					dst[d] = fo;
-					if (d == 0) {
-						dst[D] = fm;
-						dst[D + 1] = fs;
-					}
-				} else {
-					u32 const dst = map_to_cta(smem_u32(partials + split * (D + 2)), 0);
-					st_cluster_f32(dst + d * 4, fo);
-					if (d == 0) {
-						st_cluster_f32(dst + D * 4, fm);
-						st_cluster_f32(dst + D * 4 + 4, fs);
-					}
+			if constexpr (CLUSTER) {
+				u32 const dst = map_to_cta(smem_u32(partials + split * (D + 2)), 0);
+				st_cluster_f32(dst + d * 4, fo);
+				if (d == 0) {
+					st_cluster_f32(dst + D * 4, fm);
+					st_cluster_f32(dst + D * 4 + 4, fs);
+				}
+			} else if (p.n_splits > 1) {
+				f32 *dst = p.scratch + ((u64(batch) * p.n_heads + head) * p.n_splits + split) * (D + 2);
+				dst[d] = fo;
+				if (d == 0) {
+					dst[D] = fm;
+					dst[D + 1] = fs;
 				}
 			}
 		}
 	}
 	pdl_launch_dependents();   // not earlier: a next decode's clusters would be packed onto the few SMs with room
-	if (p.n_splits > 1) {
-		if (p.scratch != nullptr) return;
+	if constexpr (CLUSTER) {
 		__syncwarp();
 		cluster_arrive();              // this CTA's partials are stored
 		if (blockIdx.z != 0) return;   // its slot is free for the next CTA: only the first CTA waits
 		cluster_wait();
+	} else if (p.n_splits > 1) {
+		return;
 	}
 	// ---- the sink token: exact int32 q . sink_k, from the lanes of one row ----
 	i32 sdot = __dp4a(i32(sk.x), i32(qw[0]), 0);
@@ -318,7 +331,7 @@ attn_decode_kernel(const DecodeParams p) {
 	for (u32 mask = 1; mask < LPR; mask <<= 1) sdot += __shfl_xor_sync(0xffffffffu, sdot, mask);
 	f32 const sink_s = __fmul_rn(__int2float_rn(sdot), temp);
 	if (threadIdx.x < D) {
-		if (p.n_splits > 1) merge_partials<D>(partials, p.n_splits, threadIdx.x, fm, fs, fo);
+		if constexpr (CLUSTER) merge_partials<D>(partials, p.n_splits, threadIdx.x, fm, fs, fo);
 		decode_finish<D>(p, batch, head, threadIdx.x, fm, fs, fo, sink_s, sink_v);
 	}
 }
