@@ -34,6 +34,13 @@ def test_decode_split_forms(stream, D, kv_len, W, splits):
         assert np.max(np.abs(l.cpu().numpy() - ref_l)) <= 1e-3
 
 
+# one and two steps of keys (nothing loaded ahead), one key more (loaded ahead), in one split and over a cluster
+@pytest.mark.parametrize("D,kv_len,splits", [(128, 128, 1), (128, 257, 1), (128, 258, 1), (64, 513, 1), (64, 514, 1), (32, 1025, 1),
+                                             (32, 1026, 1), (128, 2048, 7), (128, 2048, 8), (64, 1538, 2), (128, 2048, 11), (64, 2048, 70)])
+def test_decode_steps(stream, D, kv_len, splits):
+    test_decode_split_forms(stream, D, kv_len, 0, splits)
+
+
 @pytest.mark.parametrize("D,splits", [(32, 2), (64, 8), (128, 3), (128, 8), (128, 40)])
 def test_decode_splits_without_keys(stream, D, splits):
     """A ragged batch of lengths 0 to 33: most splits have no key at all and their CTAs reach the merge before the first

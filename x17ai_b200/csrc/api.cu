@@ -604,9 +604,7 @@ SplitPlan plan_split(size_t rows, size_t n_raw, size_t k, bool f8, uint32_t head
 	x17::SplitParams &sp = plan.sp;
 	sp.tiles_m = uint32_t(tiles_m);
 	sp.a_rows = rows >= BM ? BM : uint32_t((rows + 7) / 8 * 8);
-	// three stages of up to 36 KB leave room for two CTAs per SM
-	sp.stages = sp.a_rows <= 32 ? 3 : SPLIT_MAX_STAGES;
-	// as many CTAs per tile as the SMs hold (clusters of three, or of eight, leave SMs of a GPC unused: a second wave),
+	// as many CTAs per tile as the SMs hold, one to an SM (clusters of three, or of eight, leave SMs of a GPC unused: a second wave),
 	// each with two K blocks or more (eight where whole heads are finished by one CTA)
 	size_t const least = head_dim != 0 ? 8 : 2;
 	size_t split = SPLIT_MAX;
@@ -615,10 +613,10 @@ SplitPlan plan_split(size_t rows, size_t n_raw, size_t k, bool f8, uint32_t head
 	for (;; split /= 2) {
 		sp.split = uint32_t(split);
 		sp.slots = deal_chunks(sp, head_dim);
-		if (split == 1 || (split - 1) * sp.slots * sp.a_rows * 128 <= size_t(sp.stages) * (sp.a_rows * BK + B_BYTES)) break;
+		if (split == 1 || (split - 1) * sp.slots * sp.a_rows * 128 <= size_t(SPLIT_STAGES) * (sp.a_rows * BK + B_BYTES)) break;
 	}
 	plan.grid = uint32_t(tiles * split);
-	plan.smem = split_smem_bytes(sp.a_rows, sp.stages);
+	plan.smem = split_smem_bytes(sp.a_rows);
 	return plan;
 }
 
@@ -627,7 +625,7 @@ cudaError_t gemm_go_split_kind(StreamScope const &on, SplitPlan const &plan, cud
 							   x17::GemmParams const &p) {
 	using namespace x17::gemm_cfg;
 	constexpr Kernel<&x17::gemm_split_kernel<EPI, F8>> kernel{};
-	cudaError_t const ce = allow_smem(kernel, on, split_smem_bytes(BM, SPLIT_MAX_STAGES));
+	cudaError_t const ce = allow_smem(kernel, on, split_smem_bytes(BM));
 	if (ce != cudaSuccess) return ce;
 	return launch(kernel, dim3(plan.grid), THREADS, plan.smem, stream, dim3(plan.sp.split), ta, tb, p, plan.sp);
 }

@@ -13,7 +13,7 @@
 //               overlaps the main loop of tile i+1
 //   warps 2..5  epilogue: tcgen05.ld (thread = row, registers = columns), fused math, 16-byte
 //               global stores
-// and the same roles as a pair of CTAs on two SMs (gemm_pair_kernel, the library's default): one
+// and the same roles as a pair of CTAs on two SMs (gemm_pair_kernel, the library's choice where there are rows to fill it): one
 // tcgen05.mma.cta_group::2 of M 256, N 256 per K step, issued by the pair's first CTA; each CTA loads its 128 rows
 // of A and half of the tile's rows of B and runs the epilogue of its own 128 rows.
 // Tiles are walked in groups of row tiles (row tiles fastest inside a group) so that the CTAs running together
@@ -468,7 +468,6 @@ X17_DEV void gemm_body(CUtensorMap const *tm_a_ptr, CUtensorMap const *tm_b_ptr,
 struct SplitParams {
 	u32 split;     // CTAs per tile = cluster size: 1, 2 or 4
 	u32 a_rows;    // rows of A's box: a multiple of 8, at most 128
-	u32 stages;    // ring stages of a_rows * BK + B_BYTES
 	u32 tiles_m;
 	u32 slots;     // chunks of one other CTA that the ring has room for
 	// Which CTA of the cluster finishes chunk c of a tile (four bits per chunk), and how many of the chunks before c
@@ -481,14 +480,14 @@ struct SplitParams {
 namespace gemm_cfg {
 constexpr u32 SPLIT_CHUNKS = BN / 32;
 constexpr u32 SPLIT_MAX = 4;
-constexpr u32 SPLIT_MAX_STAGES = 4;
-constexpr u32 split_smem_bytes(u32 a_rows, u32 stages) {
-	return stages * (a_rows * BK + B_BYTES) + 1024 /*alignment slack*/ + 256 /*barriers*/;
+constexpr u32 SPLIT_STAGES = 4;   // of a_rows * BK + B_BYTES: one CTA per SM
+constexpr u32 split_smem_bytes(u32 a_rows) {
+	return SPLIT_STAGES * (a_rows * BK + B_BYTES) + 1024 /*alignment slack*/ + 256 /*barriers*/;
 }
 }  // namespace gemm_cfg
 
 template <int EPI, bool F8>
-__global__ void __launch_bounds__(gemm_cfg::THREADS, 2)
+__global__ void __launch_bounds__(gemm_cfg::THREADS, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b, const GemmParams p,
 				  const SplitParams sp) {
 	using namespace gemm_cfg;
@@ -498,10 +497,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 	u32 const smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
 	u8 *const smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
 	u32 const stage_bytes = sp.a_rows * BK + B_BYTES;
-	u32 const bar_base = smem_base + sp.stages * stage_bytes;
+	u32 const bar_base = smem_base + SPLIT_STAGES * stage_bytes;
 	auto full_bar = [&](u32 s) { return bar_base + 8 * s; };
-	auto empty_bar = [&](u32 s) { return bar_base + 8 * (SPLIT_MAX_STAGES + s); };
-	u32 const acc_full_bar = bar_base + 8 * (2 * SPLIT_MAX_STAGES);
+	auto empty_bar = [&](u32 s) { return bar_base + 8 * (SPLIT_STAGES + s); };
+	u32 const acc_full_bar = bar_base + 8 * (2 * SPLIT_STAGES);
 	u32 const tmem_slot = acc_full_bar + 8;
 	volatile u32 *const tmem_slot_gen = reinterpret_cast<volatile u32 *>(smem_gen + (tmem_slot - smem_base));
 	volatile u32 *const abort_flag = tmem_slot_gen + 1;
@@ -517,7 +516,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 	u32 const kb_begin = rank * k_blocks / sp.split, kb_end = (rank + 1) * k_blocks / sp.split;
 
 	if (threadIdx.x == 0) {
-		for (u32 s = 0; s < sp.stages; ++s) {
+		for (u32 s = 0; s < SPLIT_STAGES; ++s) {
 			mbar_init(full_bar(s), 1);
 			mbar_init(empty_bar(s), 1);
 		}
@@ -533,7 +532,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 		// the first weights start on their way to L2 while the kernel in front of this one finishes
 		tma_prefetch_desc(&tm_a);
 		tma_prefetch_desc(&tm_b);
-		for (u32 i = 0; i < 2 * sp.stages && kb_begin + i < kb_end; ++i) tma_prefetch_2d(&tm_b, i32((kb_begin + i) * BK), i32(n0));
+		for (u32 i = 0; i < 2 * SPLIT_STAGES && kb_begin + i < kb_end; ++i) tma_prefetch_2d(&tm_b, i32((kb_begin + i) * BK), i32(n0));
 	}
 	tc_fence_before();
 	__syncthreads();
@@ -551,7 +550,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 				mbar_expect_tx(full_bar(s), stage_bytes);
 				tma_load_2d(a_dst + sp.a_rows * BK, &tm_b, full_bar(s), i32(kb * BK), i32(n0));
 				tma_load_2d(a_dst, &tm_a, full_bar(s), i32((kb * BK) % p.k_a), i32(m0));
-				if (++s == sp.stages) {
+				if (++s == SPLIT_STAGES) {
 					s = 0;
 					ph ^= 1;
 				}
@@ -578,7 +577,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 					else mma_i8_ss(tmem_base, adesc + 2 * ks, bdesc + 2 * ks, idesc, accumulate);
 				}
 				tc_commit(empty_bar(s));
-				if (++s == sp.stages) {
+				if (++s == SPLIT_STAGES) {
 					s = 0;
 					ph ^= 1;
 				}
