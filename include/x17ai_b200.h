@@ -261,17 +261,20 @@ enum { X17AI_B200_ATTN_PERSISTENT = 0, X17AI_B200_ATTN_PER_TILE = 1 };
 int x17ai_b200_set_attn_schedule(int schedule, unsigned tiles_per_item);
 
 /* Tiling of x17ai_b200_gemm_fwd and x17ai_b200_qkvg_fwd_i8:
- *   X17AI_B200_GEMM_AUTO (default): chosen per launch: K split over a cluster of up to eight CTAs per 128 x 256 tile
- *     for up to 128 rows, and for more rows while the CTA-pair form's tiles would keep no more than half of the SMs
- *     busy; the CTA-pair form otherwise.
+ *   X17AI_B200_GEMM_AUTO (default): chosen per launch, by shape. Up to 48 rows: the weights on the MMA's 128-row side,
+ *     K split over a cluster of up to four CTAs per 128 columns. Up to 128 rows: K split over a cluster of up to four CTAs
+ *     per 128 x 256 tile; the same for more rows while the CTA-pair form's tiles would keep no more than half of the SMs
+ *     busy. Both only where K is long enough to pay for the exchange of the parts (more rows: from 4096 on). The two forms
+ *     below otherwise.
  *   X17AI_B200_GEMM_CTA_PAIR: clusters of two CTAs on two SMs, 256 x 256 tiles
  *     (tcgen05.mma.cta_group::2): every CTA loads its 128 rows of A and half of the tile's rows of B, a third fewer
  *     bytes per MMA through L2 and shared memory, six ring stages instead of four. Taken for inputs of more than
  *     128 rows whose N is a multiple of 256; other shapes run the one-CTA form.
  *   X17AI_B200_GEMM_ONE_CTA: one CTA per SM, 128 x 256 tiles (tcgen05.mma.cta_group::1), the form the kernel
  *     objects embed (the reference's launch path has no clusters).
- * The same bytes out (f32 accumulators of the split form are added up in parts: where a sum is not exact in f32, a
- * code on a rounding tie may differ). Process-wide; returns 0, or -1 for an unknown value. */
+ * int8 x int8 gives the same bytes in every form. The f32 accumulators of the e4m3 kinds are added up in parts where K is
+ * split: where a sum is not exact in f32, a code on a rounding tie may differ from the other forms', so under AUTO a row's
+ * bytes may depend on how many rows it is batched with; the two explicit forms do not split K. Process-wide; returns 0, or -1 for an unknown value. */
 enum { X17AI_B200_GEMM_ONE_CTA = 0, X17AI_B200_GEMM_CTA_PAIR = 1, X17AI_B200_GEMM_AUTO = 2 };
 int x17ai_b200_set_gemm_tiling(int tiling);
 
@@ -291,9 +294,10 @@ x17ai_DiagnosticBuffer *x17ai_b200_attn_fwd_i8_debug(
  *   q [batch][q_stride]; kv_cache [batch][kv_capacity][kv_stride]; kv_lens [batch] or NULL
  *   (then every sequence has kv_len cached tokens); out [batch][o_stride]; l [batch][n_heads]
  *   or NULL.
- * When batch*n_heads is too small to fill the GPU the keys are split over several CTAs and
- * the partial results pass through stream-ordered scratch memory that this call allocates
- * and frees (cudaMallocAsync / cudaFreeAsync on `stream`).
+ * When batch*n_heads is too small to fill the GPU the keys are split over several CTAs. Up to 64
+ * splits the partial results meet in the shared memory of a cluster; beyond that they pass through
+ * stream-ordered scratch memory that this call allocates and frees (cudaMallocAsync /
+ * cudaFreeAsync on `stream`) and a second kernel merges them.
  */
 x17ai_DiagnosticBuffer *x17ai_b200_attn_decode_i8(
 	x17ai_CudaStreamHandle *stream, x17ai_AttnConfig const *cfg, size_t batch,
@@ -306,16 +310,17 @@ x17ai_DiagnosticBuffer *x17ai_b200_attn_decode_i8(
  * reference. Some hosts of this library run where device memory cannot be allocated at call
  * time: inside a serving loop whose memory was carved up front and handed out by the host's own
  * allocator, under a CUDA memory pool that is exhausted or disabled, or in a process whose
- * policy forbids cudaMalloc / cudaMallocAsync after start-up. For them the split-KV partials
- * go to a 4 MiB array built into the library image (every GPU that loads the library holds it
- * until the process exits) instead of stream-ordered scratch.
+ * policy forbids cudaMalloc / cudaMallocAsync after start-up. For them the partials of more than
+ * 64 splits go to a 4 MiB array built into the library image (every GPU that loads the library
+ * holds it until the process exits) instead of stream-ordered scratch.
  *   - Arguments and results are those of x17ai_b200_attn_decode_i8.
  *   - Limit: batch * n_heads * n_splits * (head_dim + 2) <= 1,048,576 floats; larger requests are
- *     rejected with a diagnostic (pass a smaller n_splits, or use the allocating entry point).
- *   - The first call on each device resolves the array's device address (cudaGetSymbolAddress
- *     with that device current); make that first call before any stream capture.
- *   - All calls share the one array: two calls whose kernels may overlap on the GPU (different
- *     streams, or different threads) race on it. Calls on one stream are safe: each call
+ *     rejected with a diagnostic, whether or not they would use the array (pass a smaller n_splits, or
+ *     use the allocating entry point).
+ *   - The first call in each context resolves the array's device address (cudaGetSymbolAddress
+ *     with that context current); make that first call before any stream capture.
+ *   - Above 64 splits all calls share the one array: two such calls whose kernels may overlap on the
+ *     GPU (different streams, or different threads) race on it. Calls on one stream are safe: each call
  *     overwrites every slot it later reads, so nothing has to be cleared between calls.
  *   - It calls no cudaMalloc, cudaFree, cudaMallocAsync or other allocating routine.
  */

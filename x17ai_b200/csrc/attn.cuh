@@ -108,7 +108,7 @@ X17_DEV f32 largest_score(f32 t, f32 a) {
 // and since the words are plain small numbers one packed fma by 2^16 puts two of four bytes in place, where the
 // 1.5 * 2^23 trick needs three byte permutes. (That wants bytes: a word of 256 in the upper place would change the lower
 // one; see largest_score.) Subnormal operands cost the packed instructions nothing.
-// Together with the bit masks above: 8 x 32 heads x 8192 x 128, window 1024 1141 -> 1095 us, 2 x 64 x 8192 x 64 522 -> 500,
+// Together with the bit masks above: 8 x 32 heads x 8192 x 128, window 1024 1141 -> 1095 us (1240 -> 1207 on another GPU), 2 x 64 x 8192 x 64 522 -> 500,
 // 2 x 64 x 2000 x 32, window 512 85.1 -> 80.7, 64 x 16384 x 32 without a window 3165 -> 3134.
 // FP8: P is written as OCP e4m3 of 256 * p instead of u8 of 255 * p.
 template <bool EDGE, bool FP8 = false, u32 N = 32>

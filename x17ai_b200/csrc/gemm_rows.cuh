@@ -5,7 +5,7 @@
 // the weights are the MMA's 128-row side, the tokens its N (16 .. 48 columns), so a K block of 128 weight rows costs
 // 16 KB of weights, the tokens' few KB and a few dozen MMA cycles, and the accumulator is a few TMEM columns. A cluster of
 // up to four CTAs splits K; the parts are exchanged through the cluster's shared memory (no workspace, no second
-// launch) and added up in K order. Small CTAs (shared memory for two or three per SM) keep enough bytes in flight
+// launch) and added up in K order. Small CTAs (shared memory for two per SM) keep enough bytes in flight
 // on every SM although the tile counts do not divide evenly.
 //
 // Epilogue: thread = output column (weight row), registers = tokens. Gate and value of a pair sit in neighbouring

@@ -71,11 +71,12 @@ X17_DEV bool elect_one() {
 	return pred != 0;
 }
 
-// Programmatic dependent launch. Every kernel of the library calls pdl_launch_dependents() once its CTA holds what it
-// allocates (TMEM: a dependent CTA on the same SM that took the columns first and then waited for this grid would wait
-// for ever), and pdl_wait() before its first access to global memory: the next kernel's set-up (launch, barriers, TMEM,
-// descriptor fetches) then runs under the tail of this one, and no kernel touches data before the grids in front of it
-// have completed. Without the launch attribute both are no-ops. A kernel's lifetime therefore begins before its inputs
+// Programmatic dependent launch. Every kernel of the library (but the one-time weight split) calls pdl_launch_dependents()
+// once its CTA holds the TMEM that it allocates (a dependent CTA on the same SM that took the columns first and then waited
+// for this grid would wait for ever), decode at its end, and pdl_wait() before its first access to global memory: the next
+// kernel's set-up (launch, barriers, TMEM, descriptor fetches) then runs under the tail of this one, and no kernel touches
+// data before the grids in front of it have completed. CTAs of one cluster start up to a microsecond apart then: whatever one
+// does to the other's shared or tensor memory comes behind a cluster barrier. Without the launch attribute both are no-ops. A kernel's lifetime therefore begins before its inputs
 // are written: they are read with plain loads or TMA, never with read-only (non-coherent) loads, which want data that
 // nobody writes while the kernel lives and which the compiler may move above the wait.
 X17_DEV void pdl_launch_dependents() {
@@ -421,7 +422,6 @@ X17_DEV void tmem_ld_32x32b_x32(u32 taddr, u32 (&r)[32]) {
 		: "memory");
 }
 
-// 32 lanes x 16 columns
 // 16 lanes x 32 columns: r[4 j + 2 h + b] is lane `thread` / 4 + 8 h, column 8 j + 2 (`thread` % 4) + b
 X17_DEV void tmem_ld_16x256b_x4(u32 taddr, u32 (&r)[16]) {
 	asm volatile(
@@ -433,6 +433,7 @@ X17_DEV void tmem_ld_16x256b_x4(u32 taddr, u32 (&r)[16]) {
 		: "r"(taddr)
 		: "memory");
 }
+// 32 lanes x 16 columns
 X17_DEV void tmem_ld_32x32b_x16(u32 taddr, u32 (&r)[16]) {
 	asm volatile(
 		"tcgen05.ld.sync.aligned.32x32b.x16.b32 "

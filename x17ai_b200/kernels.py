@@ -91,7 +91,9 @@ GEMM_ONE_CTA, GEMM_CTA_PAIR, GEMM_AUTO = 0, 1, 2
 def set_gemm_tiling(tiling: int = GEMM_AUTO) -> None:
     """Process-wide tiling of GemmKernel.launch and qkvg_fwd (x17ai_b200_set_gemm_tiling): clusters of two CTAs with
     256 x 256 tiles (tcgen05.mma.cta_group::2), one CTA per SM with 128 x 256 tiles, or (default) chosen per launch
-    between the CTA pairs and, for few rows, K split over a cluster."""
+    between these and, for few rows, K split over a cluster (128 x 256 tiles, or up to 48 rows the weights on the
+    MMA's 128-row side). int8 gives the same bytes in every form; with e4m3 activations a row's bytes may depend, on
+    rounding ties, on how many rows it is batched with where K is split."""
     if _lib.load().x17ai_b200_set_gemm_tiling(int(tiling)) != 0:
         raise X17Error(f"unknown GEMM tiling {tiling}")
 

@@ -7,7 +7,9 @@ are independent, so the units of work are independent:
   attention / decode : (sequence, head) units - sequences are split first, so that q and kv of a
                        sequence stay on one GPU; if there are fewer sequences than ranks, the heads
                        of a sequence are split into contiguous column blocks
-  GEMM / RMSNorm     : contiguous token-row blocks, rounded to the M tile; weights replicated
+  GEMM / RMSNorm     : contiguous token-row blocks, rounded to the M tile; weights replicated. (A row's int8 x int8
+                       bytes do not depend on the partition; with e4m3 activations, blocks small enough for the
+                       GEMM forms that split K may give another code on a rounding tie.)
 
 No data moves between ranks inside the path. `gather_rows` / `gather_attn` collect outputs on
 every rank (torch.distributed all_gather: NCCL on GPUs, gloo in the CPU tests) for a consumer that
